@@ -1565,7 +1565,7 @@ __device__ bool start_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
 // ---------------------------------------------------------------------------
 // Solve one instance with the CTAs of one team.  I refers to kernel-parameter
 // space (single-instance launches) or to a shared-memory copy (batches).
-template <int BS>
+template <int BS, bool LEAN>
 __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS>& sm, uint32_t* bar,
                                uint32_t& bar_epoch, uint32_t rank, uint32_t team_size, bool& inject) {
   constexpr int NW = BS / 32;
@@ -1615,14 +1615,14 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     C.heavy_ctr = &ctr->heavy[it % 3];
     C.hcap = hhalf;
     C.hitem = I.hitem + ((it & 1) ? I.icap : 0);
-    C.split = (I.light_heavy && delta != 0) ? delta : 0u;
-    C.heavy_iter = heavy_it;
-    C.sq = (C.split != 0u && !heavy_it) ? I.sq[hg & 1] : nullptr;
+    C.split = (!LEAN && I.light_heavy && delta != 0) ? delta : 0u;
+    C.heavy_iter = !LEAN && heavy_it;
+    C.sq = (!LEAN && C.split != 0u && !heavy_it) ? I.sq[hg & 1] : nullptr;
     C.sq_tail = &ctr->stail[hg % 3];
     C.sstamp = base + hg + 1;
     C.sadd = &ctr->sadd[it % 3];
-    C.local_rounds = heavy_it ? 0 : I.local_rounds;  // a heavy pass only relaxes heavy edges
-    C.order_deg = I.order_degree;
+    C.local_rounds = LEAN || heavy_it ? 0 : I.local_rounds;  // a heavy pass only relaxes heavy edges
+    C.order_deg = LEAN ? 0 : I.order_degree;
     C.ring = false;  // queues and lists of the iteration schedule
     level_thresholds(level, I.t1, I.t2, I.t3, C.t_warp, C.t_block, C.t_grid);
     // push-time sorting into the grid-tier list: plain iterations at the grid level
@@ -1854,7 +1854,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
         const uint32_t hn0 = min((uint32_t)(h1 >> kHeavyShift), hhalf);
         // an advance follows only when no heavy pass does (the far-pile length is stable only
         // then: a light or heavy pass may already be pushing to it in a faster CTA)
-        const bool heavy0 = I.light_heavy && delta != 0 && min(s_gen + s1, I.qcap) != 0;
+        const bool heavy0 = !LEAN && I.light_heavy && delta != 0 && min(s_gen + s1, I.qcap) != 0;
         const bool adv0 = qn0 == 0 && hn0 == 0 && !heavy0 && fl0 != 0;
         float hs = 0.f;
         for (int b = 0; b < 8; ++b) hs += (float)hb[b];
@@ -1904,7 +1904,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     // entries of the current settle list: every CTA adds the same per-iteration counts
     s_gen += sm.bc_s;
     const uint32_t sn = min(s_gen, I.qcap);
-    const bool split_now = I.light_heavy && delta != 0;
+    const bool split_now = !LEAN && I.light_heavy && delta != 0;
     heavy_it = false;
     if (qn == 0 && hn == 0 && split_now && sn != 0) {
       // bucket drained: relax the heavy edges of every vertex it settled, once
@@ -2367,10 +2367,11 @@ constexpr int kMinBlocks = BS >= 512 ? 2 : (BS >= 256 ? 3 : 6);
 
 // The persistent kernel.  SINGLE: one instance whose descriptor is the kernel
 // parameter `single` (constant-bank reads in the hot loops); otherwise the
-// team's instances are staged one at a time in shared memory.  ASYNC (single
+// team's instances are staged one at a time in shared memory.  LEAN: without the
+// optional orderings (nps_lean).  ASYNC (single
 // instances only): the asynchronous bucket schedule, in a kernel of its own so
 // that each schedule gets its own register allocation.
-template <int BS, bool SINGLE, bool ASYNC = false>
+template <int BS, bool SINGLE, bool ASYNC = false, bool LEAN = false>
 __global__ void __launch_bounds__(BS, kMinBlocks<BS>) sssp_persistent_kernel(const __grid_constant__ LaunchParams P,
                                                              const __grid_constant__ InstDesc single) {
   __shared__ Smem<BS> sm;
@@ -2399,13 +2400,13 @@ __global__ void __launch_bounds__(BS, kMinBlocks<BS>) sssp_persistent_kernel(con
   if constexpr (SINGLE && ASYNC) {
     solve_instance_async<BS>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
   } else if constexpr (SINGLE) {
-    solve_instance<BS>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
+    solve_instance<BS, LEAN>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
   } else {
     for (int k = 0; k < td.inst_count; ++k) {
       __syncthreads();
       if (threadIdx.x == 0) sinst = P.inst[P.order[td.inst_begin + k]];
       __syncthreads();
-      solve_instance<BS>(P, sinst, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
+      solve_instance<BS, LEAN>(P, sinst, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
       if (ld_relaxed_u32(P.abort_flag)) return;
       // instances of a team are separated by a barrier so every CTA sees the previous one done
       if (!team_barrier<BS>(P, sm, bar, bar_epoch, (uint32_t)td.cta_count, &sinst.ctr->status, false)) return;

@@ -151,17 +151,18 @@ nps_status device_info(int dev, DevInfo* out) {
 
 using KernelFn = void (*)(const LaunchParams, const InstDesc);
 
-KernelFn pick_kernel(int bs, bool single, bool async = false) {
+template <int BS>
+KernelFn pick_kernel_bs(bool single, bool async, bool lean) {
+  if (async) return nps::sssp_persistent_kernel<BS, true, true>;
+  if (single) return lean ? nps::sssp_persistent_kernel<BS, true, false, true> : nps::sssp_persistent_kernel<BS, true>;
+  return lean ? nps::sssp_persistent_kernel<BS, false, false, true> : nps::sssp_persistent_kernel<BS, false>;
+}
+
+KernelFn pick_kernel(int bs, bool single, bool async, bool lean) {
   switch (bs) {
-    case 128:
-      return async ? nps::sssp_persistent_kernel<128, true, true>
-                   : (single ? nps::sssp_persistent_kernel<128, true> : nps::sssp_persistent_kernel<128, false>);
-    case 256:
-      return async ? nps::sssp_persistent_kernel<256, true, true>
-                   : (single ? nps::sssp_persistent_kernel<256, true> : nps::sssp_persistent_kernel<256, false>);
-    case 512:
-      return async ? nps::sssp_persistent_kernel<512, true, true>
-                   : (single ? nps::sssp_persistent_kernel<512, true> : nps::sssp_persistent_kernel<512, false>);
+    case 128: return pick_kernel_bs<128>(single, async, lean);
+    case 256: return pick_kernel_bs<256>(single, async, lean);
+    case 512: return pick_kernel_bs<512>(single, async, lean);
     default: return nullptr;
   }
 }
@@ -195,8 +196,8 @@ cudaError_t set_carveout(int dev, KernelFn k, int bs, int nb) {
 }
 
 nps_status grid_size(int dev, const DevInfo& di, int bs, bool single, int ctas_per_sm, int* grid,
-                     bool async = false) {
-  KernelFn k = pick_kernel(bs, single, async);
+                     bool async, bool lean) {
+  KernelFn k = pick_kernel(bs, single, async, lean);
   if (!k) return nps_fail(NPS_ERR_INVALID_ARG, "block_size must be 128, 256 or 512");
   int nb = 0;
   NPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void*)k, bs, 0));
@@ -508,9 +509,9 @@ unsigned long long run_budget_ns(const nps_params& p) {
   return (unsigned long long)(std::max(60.0, 30.0 * p.timeout_s) * 1e9);
 }
 
-nps_status launch(nps_ctx* c, cudaStream_t s, int bs, bool single, int grid, const LaunchParams& lp,
+nps_status launch(nps_ctx* c, cudaStream_t s, int bs, bool single, bool lean, int grid, const LaunchParams& lp,
                   const InstDesc& inst) {
-  KernelFn k = pick_kernel(bs, single, single && inst.async != 0);
+  KernelFn k = pick_kernel(bs, single, single && inst.async != 0, lean);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)bs);
@@ -557,7 +558,7 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   nps_heavy_items(m, hcap / 2, 0, &icap, &ishift);
   if ((e = c->heavy.ensure(nps_heavy_slots(hcap, icap), false, s))) return e;
   int grid = 0;
-  if ((e = grid_size(c->device, c->di, p.block_size, true, p.ctas_per_sm, &grid, use_async(p)))) return e;
+  if ((e = grid_size(c->device, c->di, p.block_size, true, p.ctas_per_sm, &grid, use_async(p), nps_lean(p)))) return e;
   Control ctl(1, 1, grid);
   if ((e = c->control.ensure(ctl.bytes(), false, s))) return e;
   ctl.base = c->control.p;
@@ -653,7 +654,7 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s));
   NPS_CUDA(cudaMemcpyAsync(d_team, &td, sizeof(td), cudaMemcpyHostToDevice, s));
   if (time_it) NPS_CUDA(cudaEventRecord(c->ev[1], s));
-  if ((e = launch(c, s, p.block_size, true, grid, lp, d))) return e;
+  if ((e = launch(c, s, p.block_size, true, nps_lean(p), grid, lp, d))) return e;
   if (time_it) NPS_CUDA(cudaEventRecord(c->ev[2], s));
   NPS_CUDA(cudaMemcpyAsync(c->h_ctr, ctl.ctr(), sizeof(Counters), cudaMemcpyDeviceToHost, s));
   if (st) st->grid_ctas = grid;
@@ -965,7 +966,7 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
   NPS_CUDA(cudaSetDevice(c->device));
   cudaStream_t s = p.stream ? (cudaStream_t)p.stream : c->stream;
   int grid = 0;
-  if ((e = grid_size(c->device, c->di, p.block_size, false, p.ctas_per_sm, &grid))) return e;
+  if ((e = grid_size(c->device, c->di, p.block_size, false, p.ctas_per_sm, &grid, false, nps_lean(p)))) return e;
 
   const bool same_set = (int)c->b_key.size() == count && c->b_grid == grid && c->b_bs == p.block_size &&
                         memcmp(c->b_key.data(), inst, sizeof(nps_instance) * count) == 0 &&
@@ -1150,7 +1151,7 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
       cudaGraph_t g = nullptr;
       NPS_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       cudaError_t ce = cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s);
-      nps_status le = ce == cudaSuccess ? launch(c, s, p.block_size, false, grid, lp, dummy) : NPS_ERR_CUDA;
+      nps_status le = ce == cudaSuccess ? launch(c, s, p.block_size, false, nps_lean(p), grid, lp, dummy) : NPS_ERR_CUDA;
       cudaError_t ee = cudaStreamEndCapture(s, &g);
       if (ce != cudaSuccess) return nps_fail(NPS_ERR_CUDA, std::string("capture memset: ") + cudaGetErrorString(ce));
       if (le) {
@@ -1169,7 +1170,7 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
     NPS_CUDA(cudaGraphLaunch(c->b_graph, s));
   } else {
     NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s));
-    if ((e = launch(c, s, p.block_size, false, grid, lp, dummy))) return e;
+    if ((e = launch(c, s, p.block_size, false, nps_lean(p), grid, lp, dummy))) return e;
   }
   NPS_CUDA(cudaEventRecord(c->ev[2], s));
   NPS_CUDA(cudaMemcpyAsync(c->h_ctr, ctl.ctr(), sizeof(Counters) * count, cudaMemcpyDeviceToHost, s));

@@ -101,11 +101,11 @@ nps_status scratch_address(int device, unsigned char** out) {
 
 using KernelFn = void (*)(const LaunchParams, const InstDesc);
 
-KernelFn pick(int bs) {
+KernelFn pick(int bs, bool lean) {
   switch (bs) {
-    case 128: return nps::sssp_persistent_kernel<128, true>;
-    case 256: return nps::sssp_persistent_kernel<256, true>;
-    case 512: return nps::sssp_persistent_kernel<512, true>;
+    case 128: return lean ? nps::sssp_persistent_kernel<128, true, false, true> : nps::sssp_persistent_kernel<128, true>;
+    case 256: return lean ? nps::sssp_persistent_kernel<256, true, false, true> : nps::sssp_persistent_kernel<256, true>;
+    case 512: return lean ? nps::sssp_persistent_kernel<512, true, false, true> : nps::sssp_persistent_kernel<512, true>;
     default: return nullptr;
   }
 }
@@ -149,7 +149,7 @@ extern "C" nps_status nps_sssp_noalloc(const int32_t* d_row_ptr, const int32_t* 
       (p.level == NPS_LEVEL_HYBRID && (p.block_threshold < p.threshold || p.grid_threshold < p.block_threshold)))
     return nps_fail(NPS_ERR_INVALID_ARG, "noalloc: invalid parameters");
   if (p.device < 0 || p.device >= kMaxDevices) return nps_fail(NPS_ERR_INVALID_ARG, "noalloc: device out of range");
-  KernelFn k = pick(p.block_size);
+  KernelFn k = pick(p.block_size, nps_lean(p));
   if (!k) return nps_fail(NPS_ERR_INVALID_ARG, "noalloc: block_size must be 128, 256 or 512");
 
   DeviceGuard guard;
