@@ -66,6 +66,21 @@ constexpr int kStripes = NPS_STRIPES;  // striped work counters (at most 32: one
 static_assert(kStripes >= 1 && kStripes <= 32, "stripes are probed one per lane");
 constexpr uint32_t kStripeMask = kStripes >= 32 ? 0xffffffffu : ((1u << kStripes) - 1u);
 constexpr int kBlockListCap = 512;     // CTA list entries (block tier)
+// CTA rounds (cta_rounds): queue entries per round (two such queues share the CTA
+// list's memory), the entries with which a CTA hands over to the team, the frontier
+// entries a CTA may be seeded with, the least it takes when there are fewer, the rounds
+// between team barriers, and the degree from which a row goes to the grid-tier list.
+// Measured on a 2048 x 2048 grid (delta 16384; ms at each value): seeds 16 / 24 / 32 / 64:
+// 17.4 / 15.7 / 15.2 / 15.4; rounds 32 / 64 / 128: 15.2 / 17.4 / 18.4 (a CTA that runs
+// ahead for long relaxes with distances that others still lower); stop 64 / 128 / 192:
+// 17.0 / 15.2 / 15.3.  List degree on R-MAT 17 (delta 32) 64 / 128 / 256 / 512:
+// 0.74 / 0.70 / 0.82 / 0.83 ms.
+constexpr int kHopCap = 256;
+constexpr int kHopStop = 128;
+constexpr uint32_t kHopSeeds = 32;
+constexpr uint32_t kHopMinSeeds = 2;
+constexpr int kHopRounds = 32;
+constexpr int32_t kHopList = 128;
 
 // Per-instance device counters.  Zeroed by the host before a launch.
 struct __align__(128) Counters {
@@ -867,6 +882,13 @@ __device__ __forceinline__ void relax_loaded(const InstDesc& I, const IterCtx& C
   relax_and_push<4>(I, C, valid, v, nd, acc, S, lane);
 }
 
+// The iteration that a CTA's rounds belong to (cta_rounds).
+struct HopArgs {
+  const int32_t* srcq;
+  uint32_t begin, end;  // this CTA's share of the frontier
+  IterCtx c;
+};
+
 // ---------------------------------------------------------------------------
 // CTA shared state
 
@@ -875,7 +897,14 @@ struct Smem {
   unsigned long long blk_ctr;  // CTA list (block tier): (entries << 32) | chunks, one atomic
   int32_t ok;
   uint32_t hist[8];
-  int4 blk[kBlockListCap];     // block-tier entries {s, e, vertex, chunk offset}
+  union {
+    int4 blk[kBlockListCap];     // block-tier entries {s, e, vertex, chunk offset}
+    int4 hop[2][kHopCap];        // CTA rounds: {vertex, distance pushed, row start, row end} of
+                                 // this round and the next
+  };
+  HopArgs hop_args;            // CTA rounds: the iteration, written by thread 0
+  uint32_t hop_n[3];           // CTA rounds: entries pushed for round r in hop_n[r % 3]
+  unsigned long long hop_acc[4];         // CTA rounds: edges, improvements, first reaches, vertices of the solve
   int32_t stage[BS / 32][3][kStage];  // per-warp append staging: [near, far, settle]
   uint32_t red[4][BS / 32];
   float feat[NPS_MLP_IN];
@@ -1386,6 +1415,251 @@ __device__ __forceinline__ void walk_item(const InstDesc& I, const IterCtx& C, c
 }
 
 // ---------------------------------------------------------------------------
+// CTA rounds: an iteration whose frontier is small against the team.  There the time
+// of an iteration is its chain of dependent memory round trips (queue, distance, edge,
+// atomicMin, stamp, queue tail, store) plus the team barrier and the decision, about
+// 19,000 cycles for a few vertices per CTA, however little each CTA has to do.  So the
+// CTA takes a contiguous share of the frontier into a queue in shared memory and
+// follows its own improvements for up to kHopRounds rounds before the team meets: a
+// round's chain is the distance and row bounds, the edges, and the atomicMin.
+//
+// A queue entry is {v, d}: the distance d that this CTA's atomicMin gave v.  The round
+// that takes it reads v's distance (a load that sees the latest value) and drops the
+// entry when the distance is below d: whoever lowered it further queued v as well.  So
+// no stamp is needed, every improvement is followed exactly once, and the scheme stays
+// label-correcting whatever the CTAs' relative progress.  Improvements at or above the
+// bucket bound go to the far pile and processed vertices to the settle list as
+// everywhere.  Rows of at least kHopList edges go to the grid-tier list at every level
+// (the near stamp keeps each there once): the whole team walks them in the next
+// iteration.  A CTA stops early when its queue is empty, or when it holds more than
+// kHopStop entries: enough for the whole team, so they go to the near queue like those
+// left after the last round.
+// Out of line, its sums in shared memory: the item loop's register allocation does not
+// pay for it.  What bounds it: the latency of a round, about 2,800 cycles for one vertex
+// (smem entry, edges beside the distance, atomicMin beside the head's row bounds, smem
+// push).  Measured (ms before -> after): 2,000-vertex path 13.6 -> 2.9; 2048 x 2048 grid,
+// delta 16384, 47.1 -> 14.3 and 4,984 -> 301 iterations; uniform 16,384 x 131,072, delta
+// 64, 0.318 -> 0.169; R-MAT 20 and 22 unchanged.
+// kHopEdges edges per lane (heads nb, weights in nd) of rows at distances du (kInf: the
+// row is skipped).  Every edge goes straight to its atomicMin: the distance check before
+// it would be one more round trip of the chain, and a small frontier has few edges.  The
+// head's row bounds are read beside it, so that the next round starts with the edges.
+// Warp-collective.
+constexpr int kHopEdges = 2;
+// The fields that a round's chain reads, in registers: the descriptor and the iteration
+// are reached through memory, and reading them again after every barrier and atomic
+// would add to each step of the chain.
+struct HopHot {
+  const int32_t* row_ptr;
+  uint32_t* dist;
+  uint32_t n, T, split;
+};
+__device__ __forceinline__ void hop_relax(const InstDesc& I, const IterCtx& C, const HopHot& H,
+                                          bool (&go)[kHopEdges],
+                                          const int32_t (&nb)[kHopEdges], uint32_t (&nd)[kHopEdges],
+                                          const uint32_t (&du)[kHopEdges], uint32_t* out_n, int4* out, Acc& acc,
+                                          Stage& S, int lane) {
+  uint32_t old[kHopEdges];
+  int32_t s[kHopEdges], e[kHopEdges];
+#pragma unroll
+  for (int j = 0; j < kHopEdges; ++j) {
+    go[j] = go[j] && du[j] < kInf && (H.split == 0u || nd[j] < H.split);
+    if (go[j]) {
+      acc.edges++;
+      nd[j] = tent(du[j], nd[j]);
+      if ((uint32_t)nb[j] >= H.n) {  // neighbour id outside [0, n): record and skip
+        atomicCAS(&I.ctr->status, 0u, (uint32_t)NPS_ERR_FORMAT);
+        go[j] = false;
+      } else if (nd[j] >= kInf) {
+        go[j] = false;
+      }
+    }
+    s[j] = go[j] ? __ldg(H.row_ptr + nb[j]) : 0;
+    e[j] = go[j] ? __ldg(H.row_ptr + nb[j] + 1) : 0;
+    old[j] = go[j] ? atomicMin(H.dist + nb[j], nd[j]) : 0u;
+  }
+  uint32_t b[kHopEdges], tot = 0;
+  bool pf[kHopEdges], far = false;
+#pragma unroll
+  for (int j = 0; j < kHopEdges; ++j) {
+    go[j] = go[j] && nd[j] < old[j];
+    if (go[j]) {
+      acc.impr++;
+      if (old[j] == kInf) acc.reached++;
+    }
+    pf[j] = go[j] && nd[j] >= H.T;
+    go[j] = go[j] && nd[j] < H.T;
+    b[j] = __ballot_sync(kFull, go[j]);
+    tot += __popc(b[j]);
+    far |= __any_sync(kFull, pf[j]);
+  }
+  if (tot) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(out_n, tot);
+    base = __shfl_sync(kFull, base, 0);
+    const bool over = base + tot > (uint32_t)kHopCap;
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int j = 0; j < kHopEdges; ++j) {
+      const uint32_t p = base + __popc(b[j] & lt);
+      base += __popc(b[j]);
+      if (go[j] && p < (uint32_t)kHopCap) {
+        out[p] = make_int4(nb[j], (int32_t)nd[j], s[j], e[j]);
+        go[j] = false;
+      }
+      if (over && go[j]) go[j] = atomicExch(I.mark + nb[j], C.snear) != C.snear;
+    }
+    if (over) stage_k<kHopEdges>(S.nbuf, S.ncnt, go, nb, C.qn, C.qn_tail, I.qcap, &I.ctr->status, lane);
+  }
+  if (far) {
+#pragma unroll
+    for (int j = 0; j < kHopEdges; ++j)
+      if (pf[j]) pf[j] = atomicExch(I.fmark + nb[j], C.sfar) != C.sfar;
+    stage_k<kHopEdges>(S.fbuf, S.fcnt, pf, nb, C.fp, C.fp_tail, I.qcap, &I.ctr->status, lane);
+  }
+}
+
+template <int BS>
+static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) {
+  constexpr uint32_t NW = BS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const HopArgs& A = sm.hop_args;
+  const IterCtx& C = A.c;
+  Stage S;
+  S.nbuf = sm.stage[warp][0];
+  S.fbuf = sm.stage[warp][1];
+  S.sbuf = sm.stage[warp][2];
+  S.ncnt = S.fcnt = S.scnt = 0;
+  S.hnext = sm.hist_next;
+  S.enext = &sm.it_acc[3];
+  uint32_t* const status = &I.ctr->status;
+  const HopHot H = {I.row_ptr, I.dist, (uint32_t)I.n, C.T, C.split};
+  const int32_t* const col = I.col;
+  const uint32_t* const wts = I.w;
+  const int32_t m = I.m;
+  int32_t* const sq = C.sq;
+  const uint32_t sstamp = C.sstamp;
+  Acc acc = {0, 0, 0, 0};
+  // seeds: distance 0 as the pushed value, which no distance is below
+  for (uint32_t i = A.begin + tid; i < A.end; i += BS) {
+    const int32_t v = __ldcg(A.srcq + i);
+    sm.hop[0][i - A.begin] = make_int4(v, 0, __ldg(I.row_ptr + v), __ldg(I.row_ptr + v + 1));
+  }
+  if (tid == 0) {
+    sm.hop_n[0] = A.end - A.begin;
+    sm.hop_n[1] = 0;
+  }
+  // rows for the grid-tier list; its capacity counts rows of at least the smallest grid
+  // threshold of the parameters
+  const int32_t t_list = max(kHopList, I.level == NPS_LEVEL_HYBRID ? I.t3 : I.t1);
+  uint32_t cnt;
+  int r = 0;
+  for (;; ++r) {
+    __syncthreads();
+    cnt = min(sm.hop_n[r % 3], (uint32_t)kHopCap);
+    if (cnt == 0 || r == kHopRounds || cnt > (uint32_t)min(kHopStop, BS)) break;
+    // read for the last time at the start of round r - 1, pushed to from round r + 1 on
+    if (tid == 0) sm.hop_n[(r + 2) % 3] = 0;
+    uint32_t* const out_n = &sm.hop_n[(r + 1) % 3];
+    int4* const out = sm.hop[(r + 1) & 1];
+    // entries spread evenly over the warps, at most one per lane
+    const uint32_t per = (cnt + NW - 1) / NW;
+    const uint32_t i = warp * per + lane;
+    if (warp * per >= cnt) continue;
+    int4 q = make_int4(0, 0, 0, 0);  // {vertex, distance pushed, row start, row end}
+    uint32_t dv = kInf;
+    if ((uint32_t)lane < per && i < cnt) {
+      q = sm.hop[r & 1][i];
+      dv = ld_relaxed_u32(H.dist + q.x);
+      if (q.z < 0 || q.w < q.z || q.w > m) {  // malformed CSR row: record and skip
+        atomicCAS(status, 0u, (uint32_t)NPS_ERR_FORMAT);
+        q.z = q.w = 0;
+      }
+    }
+    // the rows' edges, flat over the warp; long rows are listed below
+    const bool lng = q.w - q.z >= t_list;
+    const uint32_t d = lng ? 0u : (uint32_t)(q.w - q.z);
+    uint32_t incl = d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const uint32_t excl = incl - d;
+    uint32_t seen = sstamp;
+    for (uint32_t k0 = 0; k0 == 0 || k0 < total; k0 += 32 * kHopEdges) {
+      int32_t nb[kHopEdges];
+      uint32_t nd[kHopEdges], du[kHopEdges];
+      int own[kHopEdges];
+      bool go[kHopEdges];
+#pragma unroll
+      for (int j = 0; j < kHopEdges; ++j) {
+        nb[j] = 0;
+        nd[j] = 0u;
+        go[j] = false;
+        own[j] = 0;
+        if (k0 + 32 * j >= total) continue;  // the whole warp
+        const uint32_t k = k0 + 32 * j + lane;
+        int o = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+          const uint32_t x = __shfl_sync(kFull, excl, o + step);
+          if (x <= k) o += step;
+        }
+        const int32_t so = __shfl_sync(kFull, q.z, o);
+        const uint32_t eo = __shfl_sync(kFull, excl, o);
+        own[j] = o;
+        go[j] = k < total;
+        if (go[j]) {
+          const int32_t ei = so + (int32_t)(k - eo);
+          nb[j] = __ldg(col + ei);
+          nd[j] = wts ? __ldg(wts + ei) : 1u;
+        }
+      }
+      if (k0 == 0) {
+        // the distance, read beside the first edges: an entry whose vertex was lowered
+        // further since is dropped, it is queued again with that distance
+        const bool fresh = dv < kInf && dv >= (uint32_t)q.y;
+        if (!fresh) dv = kInf;
+        else acc.processed++;
+        if (sq && fresh && q.w > q.z) seen = atomicExch(I.smark + q.x, sstamp);
+        if (__any_sync(kFull, lng)) {
+          bool g = lng && fresh;
+          if (g) g = atomicExch(I.mark + q.x, C.snear) != C.snear;
+          grid_append(I, C, g, q.z, q.w, q.x, lane);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kHopEdges; ++j) du[j] = __shfl_sync(kFull, dv, own[j]);
+      hop_relax(I, C, H, go, nb, nd, du, out_n, out, acc, S, lane);
+    }
+    if (sq) {
+      const bool f[1] = {seen != sstamp};
+      const int32_t vv[1] = {q.x};
+      stage_k<1>(S.sbuf, S.scnt, f, vv, sq, C.sq_tail, I.qcap, status, lane, nullptr, nullptr, C.sadd);
+    }
+  }
+  // entries left: to the near queue
+  for (uint32_t i0 = 0; i0 < cnt; i0 += BS) {
+    const uint32_t i = i0 + tid;
+    const int32_t v[1] = {i < cnt ? sm.hop[r & 1][i].x : 0};
+    const bool f[1] = {i < cnt && atomicExch(I.mark + v[0], C.snear) != C.snear};
+    stage_k<1>(S.nbuf, S.ncnt, f, v, C.qn, C.qn_tail, I.qcap, status, lane);
+  }
+  if (S.ncnt) stage_flush(S.nbuf, S.ncnt, S.ncnt, C.qn, C.qn_tail, I.qcap, status, lane);
+  if (S.fcnt) stage_flush(S.fbuf, S.fcnt, S.fcnt, C.fp, C.fp_tail, I.qcap, status, lane);
+  if (S.scnt) stage_flush(S.sbuf, S.scnt, S.scnt, C.sq, C.sq_tail, I.qcap, status, lane, C.sadd);
+  const uint32_t a[4] = {__reduce_add_sync(kFull, acc.edges), __reduce_add_sync(kFull, acc.impr),
+                         __reduce_add_sync(kFull, acc.reached), __reduce_add_sync(kFull, acc.processed)};
+  if (lane == 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (a[j]) atomicAdd(&sm.hop_acc[j], (unsigned long long)a[j]);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Learned policy: 12 features -> 32 ReLU -> 14 logits (bf16 weights, fp32 math).
 // Evaluated redundantly by every CTA of a team on identical inputs, so every
 // CTA takes the same decision without another barrier.
@@ -1597,6 +1871,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
   uint32_t reached_total = 1;
   const uint32_t hhalf = I.hcap / 2;
   if (threadIdx.x < 8) sm.hist_next[threadIdx.x] = 0;
+  if (threadIdx.x < 4) sm.hop_acc[threadIdx.x] = 0ull;
 
   for (;;) {
     // ---- iteration set-up (identical in every CTA)
@@ -1659,6 +1934,20 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       sm.hist_next[threadIdx.x] = 0;
     }
     if (threadIdx.x < 4) sm.it_acc[threadIdx.x] = 0;
+    // A frontier of at most kHopSeeds vertices per CTA and no grid-tier rows to walk: CTA
+    // rounds.  Larger frontiers give the item loop enough to hide its latency, and rounds
+    // of many entries would be bound by one CTA's throughput.  Not for the passes over
+    // the far pile and the settle list, nor where a pass per frontier is asked for: the
+    // policy's and the trace's per-iteration statistics, degree ordering, local rounds.
+    const bool hops = !advance && !heavy_it && !want_iter && hprev_tot == 0 && C.local_rounds == 0 &&
+                      C.order_deg == 0 && qlen <= team_size * kHopSeeds;
+    if (hops && threadIdx.x == 0) {
+      const uint32_t per = max(kHopMinSeeds, (qlen + team_size - 1) / team_size);
+      sm.hop_args.srcq = I.q[it & 1];
+      sm.hop_args.begin = min(qlen, rank * per);
+      sm.hop_args.end = min(qlen, rank * per + per);
+      sm.hop_args.c = C;
+    }
     __syncthreads();
     if (threadIdx.x == 0 && it > 0 &&
         !agree_step(ctr, it - 1, team_size, &sm.agree_prev, sm.bc_ag,
@@ -1673,112 +1962,116 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
 
     const int32_t* srcq = advance ? I.fq[ep & 1] : (heavy_it ? I.sq[hg & 1] : I.q[it & 1]);
     const uint32_t srclen = advance ? adv_len : (heavy_it ? slen : qlen);
-    const uint32_t n_heavy_items = (uint32_t)((hprev_tot + (1ull << I.item_shift) - 1) >> I.item_shift);
-    // vertex items hold 32 frontier entries, or 16 / 8 / 4 when the frontier is small
-    // against the team's warps: a small frontier's rows then spread over more warps
-    // instead of leaving a few warps with 32 rows each
-    uint32_t vper = 32;
-    while (vper > 4 && (unsigned long long)srclen < (unsigned long long)vper * team_size * NW) vper >>= 1;
-    const uint32_t n_items = n_heavy_items + (srclen + vper - 1) / vper;
     Acc acc = {0, 0, 0, 0};
-    Stage S;
-    S.nbuf = sm.stage[warp][0];
-    S.fbuf = sm.stage[warp][1];
-    S.sbuf = sm.stage[warp][2];
-    S.ncnt = 0;
-    S.fcnt = 0;
-    S.scnt = 0;
-    S.fmin = 0xffffffffu;
-    S.credit = nullptr;  // ring mode only
-    S.hnext = sm.hist_next;
-    S.enext = &sm.it_acc[3];
+    if (hops) {
+      cta_rounds<BS>(I, sm);
+    } else {
+      const uint32_t n_heavy_items = (uint32_t)((hprev_tot + (1ull << I.item_shift) - 1) >> I.item_shift);
+      // vertex items hold 32 frontier entries, or 16 / 8 / 4 when the frontier is small
+      // against the team's warps: a small frontier's rows then spread over more warps
+      // instead of leaving a few warps with 32 rows each
+      uint32_t vper = 32;
+      while (vper > 4 && (unsigned long long)srclen < (unsigned long long)vper * team_size * NW) vper >>= 1;
+      const uint32_t n_items = n_heavy_items + (srclen + vper - 1) / vper;
+      Stage S;
+      S.nbuf = sm.stage[warp][0];
+      S.fbuf = sm.stage[warp][1];
+      S.sbuf = sm.stage[warp][2];
+      S.ncnt = 0;
+      S.fcnt = 0;
+      S.scnt = 0;
+      S.fmin = 0xffffffffu;
+      S.credit = nullptr;  // ring mode only
+      S.hnext = sm.hist_next;
+      S.enext = &sm.it_acc[3];
 
-    // ---- work loop: heavy chunk items, then vertex items.  With no more items than
-    // warps, warp w takes item w (no atomics); otherwise items come from striped
-    // counters, the next index requested before the current item is processed, and
-    // an exhausted stripe answered by a parallel probe of all stripes.
-    {
-      const uint32_t team_warps = team_size * NW;
-      const bool static_items = n_items <= team_warps;
-      uint32_t* wc = &ctr->work[it % 3][0];
-      int stripe = (int)(gwarp % kStripes);
-      uint32_t t_next = 0;
-      bool have_next = false;
-      bool static_done = false;
-      for (;;) {
-        unsigned long long item;
-        if (static_items) {
-          if (static_done || gwarp >= n_items) break;
-          static_done = true;
-          item = gwarp;
-        } else {
-          uint32_t t = 0;
-          if (lane == 0) t = have_next ? t_next : atomicAdd(&wc[stripe * 32], 1u);
-          t = __shfl_sync(kFull, t, 0);
-          have_next = false;
-          const uint32_t my_items = n_items > (uint32_t)stripe ? (n_items - stripe + kStripes - 1) / kStripes : 0u;
-          if (t >= my_items) {
-            // probe every stripe at once; continue on the first one with items left
-            const uint32_t li = n_items > (uint32_t)lane ? (n_items - lane + kStripes - 1) / kStripes : 0u;
-            const bool avail = lane < kStripes && ld_relaxed_u32(&wc[lane * 32]) < li;
-            const uint32_t m = __ballot_sync(kFull, avail);
-            if (m == 0) break;
-            const unsigned long long mm = (unsigned long long)m | ((unsigned long long)m << kStripes);
-            const uint32_t rot = (uint32_t)(mm >> (stripe + 1)) & kStripeMask;  // m rotated right by stripe + 1
-            stripe = (stripe + __ffs(rot)) % kStripes;
-            continue;
-          }
-          if (lane == 0) t_next = atomicAdd(&wc[stripe * 32], 1u);
-          have_next = true;
-          item = (unsigned long long)t * kStripes + stripe;
-        }
-        NPS_LAP(pc, 0);
-        if (item < n_heavy_items) {
-          const uint32_t kb = (uint32_t)item << I.item_shift;
-          const uint32_t ke = (uint32_t)min((unsigned long long)kb + (1ull << I.item_shift), hprev_tot);
-          const int32_t js = __ldcg(Hitem + item);
-          walk_item(I, C, Hprev, hprev_cnt, kb, ke, (uint32_t)js, acc, S, lane);
-          NPS_LAP(pc, 4);
-        } else {
-          const uint32_t idx = (uint32_t)(item - n_heavy_items) * vper + lane;
-          process_vertex_item<BS>(I, C, sm, ((uint32_t)lane < vper && idx < srclen) ? __ldcg(srcq + idx) : -1, advance,
-                                  T_old, want_iter, acc, S, pc, lane);
-          // warp-local rounds: vertices this warp just queued for the next iteration are
-          // taken back from its staging buffer and processed now, up to local_rounds times;
-          // their stamp is reset so a later improvement in this iteration queues them again
-          for (int r = 0; r < C.local_rounds && S.ncnt > 0; ++r) {
-            const uint32_t k = min(S.ncnt, 32u);
-            int32_t lv = -1;
-            if ((uint32_t)lane < k) {
-              lv = S.nbuf[S.ncnt - k + lane];
-              atomicExch(I.mark + lv, 0u);
-              __threadfence();  // the reset is visible before lv's distance is read
+      // ---- work loop: heavy chunk items, then vertex items.  With no more items than
+      // warps, warp w takes item w (no atomics); otherwise items come from striped
+      // counters, the next index requested before the current item is processed, and
+      // an exhausted stripe answered by a parallel probe of all stripes.
+      {
+        const uint32_t team_warps = team_size * NW;
+        const bool static_items = n_items <= team_warps;
+        uint32_t* wc = &ctr->work[it % 3][0];
+        int stripe = (int)(gwarp % kStripes);
+        uint32_t t_next = 0;
+        bool have_next = false;
+        bool static_done = false;
+        for (;;) {
+          unsigned long long item;
+          if (static_items) {
+            if (static_done || gwarp >= n_items) break;
+            static_done = true;
+            item = gwarp;
+          } else {
+            uint32_t t = 0;
+            if (lane == 0) t = have_next ? t_next : atomicAdd(&wc[stripe * 32], 1u);
+            t = __shfl_sync(kFull, t, 0);
+            have_next = false;
+            const uint32_t my_items = n_items > (uint32_t)stripe ? (n_items - stripe + kStripes - 1) / kStripes : 0u;
+            if (t >= my_items) {
+              // probe every stripe at once; continue on the first one with items left
+              const uint32_t li = n_items > (uint32_t)lane ? (n_items - lane + kStripes - 1) / kStripes : 0u;
+              const bool avail = lane < kStripes && ld_relaxed_u32(&wc[lane * 32]) < li;
+              const uint32_t m = __ballot_sync(kFull, avail);
+              if (m == 0) break;
+              const unsigned long long mm = (unsigned long long)m | ((unsigned long long)m << kStripes);
+              const uint32_t rot = (uint32_t)(mm >> (stripe + 1)) & kStripeMask;  // m rotated right by stripe + 1
+              stripe = (stripe + __ffs(rot)) % kStripes;
+              continue;
             }
-            __syncwarp();
-            S.ncnt -= k;
-            process_vertex_item<BS>(I, C, sm, lv, false, T_old, want_iter, acc, S, pc, lane, true);
+            if (lane == 0) t_next = atomicAdd(&wc[stripe * 32], 1u);
+            have_next = true;
+            item = (unsigned long long)t * kStripes + stripe;
+          }
+          NPS_LAP(pc, 0);
+          if (item < n_heavy_items) {
+            const uint32_t kb = (uint32_t)item << I.item_shift;
+            const uint32_t ke = (uint32_t)min((unsigned long long)kb + (1ull << I.item_shift), hprev_tot);
+            const int32_t js = __ldcg(Hitem + item);
+            walk_item(I, C, Hprev, hprev_cnt, kb, ke, (uint32_t)js, acc, S, lane);
+            NPS_LAP(pc, 4);
+          } else {
+            const uint32_t idx = (uint32_t)(item - n_heavy_items) * vper + lane;
+            process_vertex_item<BS>(I, C, sm, ((uint32_t)lane < vper && idx < srclen) ? __ldcg(srcq + idx) : -1, advance,
+                                    T_old, want_iter, acc, S, pc, lane);
+            // warp-local rounds: vertices this warp just queued for the next iteration are
+            // taken back from its staging buffer and processed now, up to local_rounds times;
+            // their stamp is reset so a later improvement in this iteration queues them again
+            for (int r = 0; r < C.local_rounds && S.ncnt > 0; ++r) {
+              const uint32_t k = min(S.ncnt, 32u);
+              int32_t lv = -1;
+              if ((uint32_t)lane < k) {
+                lv = S.nbuf[S.ncnt - k + lane];
+                atomicExch(I.mark + lv, 0u);
+                __threadfence();  // the reset is visible before lv's distance is read
+              }
+              __syncwarp();
+              S.ncnt -= k;
+              process_vertex_item<BS>(I, C, sm, lv, false, T_old, want_iter, acc, S, pc, lane, true);
+            }
           }
         }
       }
-    }
-    NPS_LAP(pc, 0);
-    // ---- block tier: the CTA's warps walk the CTA list once
-    __syncthreads();
-    const uint32_t bcnt = min((uint32_t)(sm.blk_ctr >> 32), (uint32_t)kBlockListCap);
-    if (bcnt) {
-      // chunks of the stored entries only (overflowed entries were walked by their warp)
-      const int4 last = sm.blk[bcnt - 1];
-      const uint32_t btot = (uint32_t)last.w + row_chunks(last.x, last.y);
-      const uint32_t per = (btot + NW - 1) / NW;
-      const unsigned long long kb = (unsigned long long)warp * per;
-      const unsigned long long ke = min((unsigned long long)btot, kb + per);
-      walk_chunks(I, C, sm.blk, bcnt, kb, ke, acc, S, lane);
+      NPS_LAP(pc, 0);
+      // ---- block tier: the CTA's warps walk the CTA list once
       __syncthreads();
-      if (threadIdx.x == 0) sm.blk_ctr = 0ull;
+      const uint32_t bcnt = min((uint32_t)(sm.blk_ctr >> 32), (uint32_t)kBlockListCap);
+      if (bcnt) {
+        // chunks of the stored entries only (overflowed entries were walked by their warp)
+        const int4 last = sm.blk[bcnt - 1];
+        const uint32_t btot = (uint32_t)last.w + row_chunks(last.x, last.y);
+        const uint32_t per = (btot + NW - 1) / NW;
+        const unsigned long long kb = (unsigned long long)warp * per;
+        const unsigned long long ke = min((unsigned long long)btot, kb + per);
+        walk_chunks(I, C, sm.blk, bcnt, kb, ke, acc, S, lane);
+        __syncthreads();
+        if (threadIdx.x == 0) sm.blk_ctr = 0ull;
+      }
+      NPS_LAP(pc, 5);
+      stage_drain(I, S, C, I.qcap, &ctr->status, lane);
+      NPS_LAP(pc, 6);
     }
-    NPS_LAP(pc, 5);
-    stage_drain(I, S, C, I.qcap, &ctr->status, lane);
-    NPS_LAP(pc, 6);
 
     // ---- iteration counters (policy features, trace): warp sums into shared
     // memory; thread 0 adds the CTA's totals to the instance counters just before
@@ -1940,10 +2233,10 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
   uint32_t r[4];
   block_sum4<BS>(sm, tot.edges, tot.impr, tot.reached, tot.processed, r);
   if (threadIdx.x == 0) {
-    atomicAdd(&ctr->edges, (unsigned long long)r[0]);
-    atomicAdd(&ctr->improvements, (unsigned long long)r[1]);
-    atomicAdd(&ctr->reached, r[2]);
-    atomicAdd(&ctr->processed, (unsigned long long)r[3]);
+    atomicAdd(&ctr->edges, (unsigned long long)r[0] + sm.hop_acc[0]);
+    atomicAdd(&ctr->improvements, (unsigned long long)r[1] + sm.hop_acc[1]);
+    atomicAdd(&ctr->reached, r[2] + (uint32_t)sm.hop_acc[2]);
+    atomicAdd(&ctr->processed, (unsigned long long)r[3] + sm.hop_acc[3]);
   }
 #ifdef NPS_PROFILE
   if (lane == 0)
