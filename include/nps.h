@@ -123,8 +123,8 @@ typedef struct nps_params {
   uint32_t delta_schedule;  /* 0: every bucket is delta wide.  Otherwise bucket b (0 = the first)
                                is 2^k wide with k = bits [4b, 4b+4) for b < 7 and bits [28, 32)
                                for every later bucket; delta is then unused (plain policy only) */
-  int32_t reserved[2];      /* reserved[0] = 1: test hook, the first in-kernel barrier (of the SSSP
-                               kernel, or of nps_color's round kernel) waits for an arrival that
+  int32_t reserved[2];      /* reserved[0] = 1: test hook, the first in-kernel wait (the SSSP kernel's
+                               barrier, or nps_color's first wait for a color) is for an arrival that
                                never comes, so its bounded wait must expire.
                                reserved[0] = 2: test hook, CTA 1 of the SSSP kernel reports another
                                hash for its first schedule decision, so the agreement check must
@@ -348,8 +348,9 @@ nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t
  * receives the colors the reference's iterations assign, color(v) = 1 + the
  * largest color among v's out-neighbours with a smaller id (1 when there is
  * none); st->iterations = the largest color (the reference's iteration count).
- * Rows of at least p->threshold edges are scanned by a warp.  Pointers are host
- * or device per p->device_ptrs; uses p->device, p->stream and p->timeout_s. */
+ * p->threshold is checked (at least 1); the kernel cuts long rows at lengths of its
+ * own.  Pointers are host or device per p->device_ptrs; uses p->device, p->stream,
+ * p->timeout_s (the bound on each wait for a color) and p->ctas_per_sm. */
 nps_status nps_color(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t m, const nps_params* p,
                      int32_t* color_out, nps_stats* st);
 
