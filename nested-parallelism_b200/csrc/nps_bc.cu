@@ -194,6 +194,339 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
   }
 }
 
+// ---- the whole source in shared memory
+//
+// Level, path count, dependency and order of every vertex of a small graph fit an SM's
+// shared memory (12 1/8 bytes per vertex).  The random accesses that bound the kernel
+// above -- an L2 sector per edge and array -- then stay on the SM, and only the edges
+// come from L2, in order.  A warp takes up to 32 vertices of the level (fewer when the
+// level is small against the CTA), a stride apart: a level's long rows come first in the
+// order, as most edges lead to them, and so spread over the items (R-MAT 14, every source:
+// 57 ms with consecutive vertices).  It walks their rows flat, so a row's length does not
+// hold a lane.  In the backward pass the lanes compute the terms of consecutive edges
+// side by side; the float sum of a row, whose order and roundings are the reference's,
+// is then formed by the lane that owns the row, from the terms in shared memory.
+//
+// What bounds it: instruction issue (ncu, R-MAT 14: 56 % of issue slots, ALU the busiest
+// pipe) and the level barriers; shared memory and L2 are below half.  Measured against the
+// kernel above: R-MAT 14, every source, 88 -> 34.4 ms; R-MAT 12 6.6 -> 2.2; uniform 6,209 x
+// 23,666 4.5 -> 3.1; 380 sources of R-MAT 12 at edge factor 4 0.72 -> 0.14.  Of that: flat
+// rows in shared memory 57 ms, items a stride apart 52, long rows without the owner search
+// 44, their sums by ordered_sum 42, heads gathered before their terms are formed 34.
+constexpr int kFwdEdges = 4;      // edges per lane and step, forward
+constexpr int kBwdEdges = 2;      // ... and backward
+constexpr int kSmemBounds = 256;  // level bounds kept in shared memory; deeper ones in a.lb
+constexpr uint16_t kUnseen = 0xffff;
+constexpr int32_t kLongRow = 32;        // rows of at least this many edges are walked one at a time
+
+// Shared memory of a CTA of `threads` for a graph of n vertices.
+__host__ __device__ constexpr size_t bc_smem_bytes(size_t n, int threads) {
+  return (size_t)(threads / 32) * 32 * kBwdEdges * sizeof(double) + n * (4 + 4) + ((n + 31) / 32) * 4 +
+         ((n + 1) & ~(size_t)1) * 4;
+}
+
+// Flat walk of one row per lane: the exclusive prefix and the total of their lengths.
+__device__ __forceinline__ uint32_t flat_prefix(uint32_t d, int lane, uint32_t& excl) {
+  uint32_t incl = d;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  excl = incl - d;
+  return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// The lane whose row holds flat position k: the last one whose prefix is <= k.
+__device__ __forceinline__ int flat_owner(uint32_t excl, uint32_t k) {
+  int o = 0;
+#pragma unroll
+  for (int step = 16; step >= 1; step >>= 1) {
+    const uint32_t x = __shfl_sync(0xffffffffu, excl, o + step);
+    if (x <= k) o += step;
+  }
+  return o;
+}
+
+// du plus the terms t of lanes 0 .. n - 1 as the reference adds them: one after the other,
+// each sum rounded to double and then to float.  One term at a time that is a chain of 51 cycles
+// per term.  While the running sum stays in one binade [2^E, 2^(E+1)) it is a multiple m u
+// of u = 2^(E-23), and adding t >= 0 gives (m + r) u: the first rounding, to multiples of
+// 2^(E-52), and the second, to multiples of u, round t itself, whatever m is, unless t
+// then lies halfway between two multiples of u (the one case that depends on m's parity).
+// So the lanes round their terms at once (adding and subtracting 1.5 2^E and 1.5 2^(E+29)
+// rounds to those multiples), a warp scan of the exact r u gives every running sum, and
+// only a term that leaves the binade, is a tie, or is not small against the sum is added
+// by itself.  Every lane returns the sum.
+__device__ __forceinline__ float ordered_sum(float du, double t, uint32_t n, int lane) {
+  constexpr unsigned kAll = 0xffffffffu;
+  uint32_t pos = 0;
+  for (int stops = 0; pos < n; ++stops) {
+    const int eb = (int)(__float_as_uint(du) >> 23);  // biased exponent; 256 or more: negative
+    if (eb < 64 || eb > 190 || stops == 8) {
+      for (uint32_t c = pos; c < n; ++c) du = __double2float_rn(__dadd_rn((double)du, __shfl_sync(kAll, t, c)));
+      break;
+    }
+    const int E = eb - 127 + 1023;  // as a double's biased exponent
+    const double k1 = __hiloint2double(E << 20 | 0x80000, 0), k2 = __hiloint2double((E + 29) << 20 | 0x80000, 0);
+    const double half = __hiloint2double((E - 24) << 20, 0), small = __hiloint2double((E - 1) << 20, 0);
+    const double top = __hiloint2double((E + 1) << 20, 0);
+    const bool in = (uint32_t)lane >= pos && (uint32_t)lane < n;
+    const double z = __dadd_rn(__dadd_rn(t, k1), -k1), r = __dadd_rn(__dadd_rn(z, k2), -k2);
+    const bool alone = in && (!(t >= 0.0 && t < small) || fabs(__dadd_rn(z, -r)) == half);
+    double p = in && !alone ? r : 0.0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double q = __shfl_up_sync(kAll, p, o);
+      if (lane >= o) p = __dadd_rn(p, q);
+    }
+    const double x = __dadd_rn((double)du, p);
+    const uint32_t b = __ballot_sync(kAll, in && (alone || !(x < top)));
+    const uint32_t f = b ? (uint32_t)__ffs(b) - 1u : n;  // terms before f are in
+    if (f > pos) du = __double2float_rn(__shfl_sync(kAll, x, f - 1));
+    if (f < n) du = __double2float_rn(__dadd_rn((double)du, __shfl_sync(kAll, t, f)));
+    pos = f + 1;
+  }
+  return du;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
+  constexpr int NW = NT / 32;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ double s_dyn[];
+  __shared__ int s_tail, s_item[2];
+  __shared__ int32_t s_lb[kSmemBounds];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int n = a.n, words = (n + 31) / 32;
+  double* const term = s_dyn + warp * 32 * kBwdEdges;    // this warp's terms of short rows,
+  int32_t* const head = reinterpret_cast<int32_t*>(term);  // or up to 95 heads of a long row
+  int32_t* const sigma = reinterpret_cast<int32_t*>(s_dyn + NW * 32 * kBwdEdges);
+  float* const delta = reinterpret_cast<float*>(sigma + n);
+  uint32_t* const seen = reinterpret_cast<uint32_t*>(delta + n);
+  uint16_t* const level = reinterpret_cast<uint16_t*>(seen + words);
+  uint16_t* const order = level + ((n + 1) & ~1);
+  int32_t* const lb = a.lb + (size_t)blockIdx.x * ((size_t)n + 2);
+  auto bound = [&](int32_t L) { return L < kSmemBounds ? s_lb[L] : __ldcg(lb + L); };
+  auto set_bound = [&](int32_t L, int32_t v) {
+    if (L < kSmemBounds) s_lb[L] = v;
+    else lb[L] = v;
+  };
+  // Forward edge to v from a vertex of level L with path count su (lanes with `on`).
+  auto reach = [&](int32_t v, int32_t su, bool on, int32_t L) {
+    if (on && (uint32_t)v >= (uint32_t)n) {
+      flag_format(a.status);
+      on = false;
+    }
+    if (!on) return;
+    uint32_t lv = level[v];
+    if (lv == kUnseen) {
+      const uint32_t bit = 1u << (v & 31);
+      if ((atomicOr(&seen[v >> 5], bit) & bit) == 0u) {  // the first edge to reach v
+        level[v] = (uint16_t)(L + 1);
+        order[atomicAdd(&s_tail, 1)] = (uint16_t)v;
+      }
+      lv = (uint32_t)L + 1u;  // whoever was first was so in this level
+    }
+    if (lv == (uint32_t)L + 1u) atomicAdd(&sigma[v], su);  // wraps as the reference's int sum does
+  };
+  // Backward: the term of edge u -> v for u of level d with path count su, stored at the
+  // lane's rank behind `base` when v is on level d + 1.  Returns who stored one.
+  auto terms = [&](int32_t v, int32_t su, int32_t d, uint32_t base) {
+    const bool on = (uint32_t)v < (uint32_t)n && level[v] == (uint32_t)d + 1u;
+    const uint32_t b = __ballot_sync(kAll, on);
+    if (on) {
+      const double r = __ddiv_rn((double)su, (double)sigma[v]);
+      term[base + __popc(b & lt)] = __dmul_rn(r, (double)__fadd_rn(1.0f, delta[v]));
+    }
+    return b;
+  };
+  for (int j = blockIdx.x; j < a.count; j += gridDim.x) {
+    const int32_t src = a.sources ? a.sources[a.src_base + j] : a.src_base + j;
+    for (int v = tid; v < n; v += NT) {
+      sigma[v] = v == src;
+      delta[v] = 0.0f;
+      level[v] = v == src ? 0 : kUnseen;
+    }
+    for (int i = tid; i < words; i += NT) seen[i] = i == src / 32 ? 1u << (src % 32) : 0u;
+    if (tid == 0) {
+      order[0] = (uint16_t)src;
+      set_bound(0, 0);
+      set_bound(1, 1);
+      s_tail = 1;
+      s_item[0] = s_item[1] = 0;
+    }
+    __syncthreads();
+    int sweep = 0;  // levels walked: the item counter of a level is reset in the next one
+    // ---- forward: the frontier is order[bound(L), bound(L + 1))
+    int32_t L = 0;
+    for (;; ++L, ++sweep) {
+      const int32_t lo = bound(L), hi = bound(L + 1);
+      if (lo >= hi) break;
+      if (tid == 0) s_item[(sweep + 1) & 1] = 0;
+      const int per = min(32, (hi - lo + NW - 1) / NW), items = (hi - lo + per - 1) / per;
+      for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(&s_item[sweep & 1], 1);
+        it = __shfl_sync(kAll, it, 0);
+        if (it >= items) break;
+        const int32_t i = lo + it + lane * items;
+        int32_t rs = 0, re = 0, su = 0;
+        if (lane < per && i < hi) {
+          const int32_t u = order[i];
+          row_ok(a, u, rs, re);
+          su = sigma[u];
+        }
+        uint32_t lng = __ballot_sync(kAll, re - rs >= kLongRow), excl;
+        const uint32_t total = flat_prefix(re - rs < kLongRow ? (uint32_t)(re - rs) : 0u, lane, excl);
+        for (uint32_t k0 = 0; k0 < total; k0 += 32 * kFwdEdges) {
+          int32_t v[kFwdEdges], s[kFwdEdges];
+#pragma unroll
+          for (int q = 0; q < kFwdEdges; ++q) {
+            v[q] = -1;
+            s[q] = 0;
+            if (k0 + 32 * q >= total) continue;  // the whole warp
+            const uint32_t k = k0 + 32 * q + lane;
+            const int o = flat_owner(excl, k);
+            const int32_t so = __shfl_sync(kAll, rs, o);
+            const uint32_t eo = __shfl_sync(kAll, excl, o);
+            s[q] = __shfl_sync(kAll, su, o);
+            if (k < total) v[q] = __ldg(a.col + so + (int32_t)(k - eo));
+          }
+#pragma unroll
+          for (int q = 0; q < kFwdEdges; ++q)
+            if (k0 + 32 * q < total) reach(v[q], s[q], k0 + 32 * q + lane < total, L);
+        }
+        // long rows, one at a time: no search for an edge's owner
+        while (lng) {
+          const int o = __ffs(lng) - 1;
+          lng &= lng - 1;
+          const int32_t so = __shfl_sync(kAll, rs, o), eo = __shfl_sync(kAll, re, o);
+          const int32_t s = __shfl_sync(kAll, su, o);
+          const int32_t* c = a.col + so + lane;
+          int32_t rest = eo - so;
+          for (; rest >= 32 * kFwdEdges; rest -= 32 * kFwdEdges, c += 32 * kFwdEdges) {
+            int32_t v[kFwdEdges];
+#pragma unroll
+            for (int q = 0; q < kFwdEdges; ++q) v[q] = __ldg(c + 32 * q);
+#pragma unroll
+            for (int q = 0; q < kFwdEdges; ++q) reach(v[q], s, true, L);
+          }
+          for (; rest > 0; rest -= 32, c += 32) reach(lane < rest ? __ldg(c) : 0, s, lane < rest, L);
+        }
+      }
+      __syncthreads();
+      if (tid == 0) set_bound(L + 2, s_tail);
+      __syncthreads();
+    }
+    // ---- backward: levels L - 2 down to 1 (as in bc_sources_kernel)
+    for (int32_t d = L - 2; d >= 1; --d, ++sweep) {
+      const int32_t lo = bound(d), hi = bound(d + 1);
+      if (tid == 0) s_item[(sweep + 1) & 1] = 0;
+      const int per = min(32, (hi - lo + NW - 1) / NW), items = (hi - lo + per - 1) / per;
+      for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(&s_item[sweep & 1], 1);
+        it = __shfl_sync(kAll, it, 0);
+        if (it >= items) break;
+        const int32_t i = lo + it + lane * items;
+        int32_t u = 0, rs = 0, re = 0, su = 0;
+        const bool own = lane < per && i < hi;
+        if (own) {
+          u = order[i];
+          rs = a.row[u];
+          re = a.row[u + 1];
+          if (rs < 0 || re < rs || (int64_t)re > a.m) rs = re = 0;  // reported in the forward pass
+          su = sigma[u];
+        }
+        uint32_t lng = __ballot_sync(kAll, re - rs >= kLongRow), excl;
+        const uint32_t deg = re - rs < kLongRow ? (uint32_t)(re - rs) : 0u;
+        const uint32_t total = flat_prefix(deg, lane, excl);
+        float du = 0.0f;
+        for (uint32_t k0 = 0; k0 < total; k0 += 32 * kBwdEdges) {
+          uint32_t b[kBwdEdges];
+          int32_t v[kBwdEdges], s[kBwdEdges];
+#pragma unroll
+          for (int q = 0; q < kBwdEdges; ++q) {
+            const uint32_t k = k0 + 32 * q + lane;
+            const int o = flat_owner(excl, k);
+            const int32_t so = __shfl_sync(kAll, rs, o);
+            const uint32_t eo = __shfl_sync(kAll, excl, o);
+            s[q] = __shfl_sync(kAll, su, o);
+            v[q] = k < total ? __ldg(a.col + so + (int32_t)(k - eo)) : -1;
+          }
+          b[0] = terms(v[0], s[0], d, 0);
+          b[1] = terms(v[1], s[1], d, __popc(b[0]));
+          __syncwarp();
+          // this lane's row: the terms of its edges in [k0, k0 + 64), in order
+          if (deg && excl < k0 + 32 * kBwdEdges && excl + deg > k0) {
+            const uint64_t on = (uint64_t)b[1] << 32 | b[0];
+            const uint32_t p0 = max(excl, k0) - k0, p1 = min(excl + deg, k0 + 32 * kBwdEdges) - k0;
+            const uint32_t c0 = __popcll(on & (((uint64_t)1 << p0) - 1));
+            const uint32_t c1 = p1 >= 64 ? __popcll(on) : __popcll(on & (((uint64_t)1 << p1) - 1));
+            for (uint32_t c = c0; c < c1; ++c) du = __double2float_rn(__dadd_rn((double)du, term[c]));
+          }
+          __syncwarp();
+        }
+        // long rows, one at a time; every lane forms the sum
+        while (lng) {
+          const int o = __ffs(lng) - 1;
+          lng &= lng - 1;
+          const int32_t so = __shfl_sync(kAll, rs, o), eo = __shfl_sync(kAll, re, o);
+          const int32_t s = __shfl_sync(kAll, su, o);
+          // heads on level d + 1 gather in order; 32 at a time the lanes form their terms
+          float dl = 0.0f;
+          uint32_t have = 0;
+          auto flush = [&](uint32_t from, uint32_t cnt) {
+            double t = 0.0;
+            if ((uint32_t)lane < cnt) {
+              const int32_t v = head[from + lane];
+              t = __dmul_rn(__ddiv_rn((double)s, (double)sigma[v]), (double)__fadd_rn(1.0f, delta[v]));
+            }
+            dl = ordered_sum(dl, t, cnt, lane);
+          };
+          const int32_t* c = a.col + so + lane;
+          int32_t rest = eo - so;
+          int32_t v0 = lane < rest ? __ldg(c) : -1, v1 = 32 + lane < rest ? __ldg(c + 32) : -1;
+          for (; rest > 0; rest -= 64) {
+            const bool on0 = (uint32_t)v0 < (uint32_t)n && level[v0] == (uint32_t)d + 1u;
+            const bool on1 = (uint32_t)v1 < (uint32_t)n && level[v1] == (uint32_t)d + 1u;
+            const uint32_t b0 = __ballot_sync(kAll, on0), b1 = __ballot_sync(kAll, on1);
+            if (on0) head[have + __popc(b0 & lt)] = v0;
+            have += __popc(b0);
+            if (on1) head[have + __popc(b1 & lt)] = v1;
+            have += __popc(b1);
+            c += 64;  // the next heads load while these are summed
+            v0 = 64 + lane < rest ? __ldg(c) : -1;
+            v1 = 96 + lane < rest ? __ldg(c + 32) : -1;
+            if (have >= 32) {
+              __syncwarp();
+              flush(0, 32);
+              if (have >= 64) flush(32, 32);
+              const uint32_t done = have & ~31u;
+              const int32_t y = head[done + lane < 96u ? done + lane : 95u];
+              __syncwarp();
+              head[lane] = y;
+              have -= done;
+            }
+          }
+          __syncwarp();
+          if (have) flush(0, have);
+          __syncwarp();
+          if (lane == o) du = dl;
+        }
+        if (own) delta[u] = du;
+      }
+      __syncthreads();
+    }
+    float* const out = a.delta + (size_t)j * n;
+    for (int v = tid; v < n; v += NT) out[v] = delta[v];
+    __syncthreads();
+  }
+}
+static_assert(kBwdEdges == 2, "two ballots make the mask of a backward step, and 128 words hold 95 heads");
+
 // bc[v] += delta_j[v] for the block's sources j in order (float, one rounding per add).
 __global__ void bc_fold_kernel(float* bc, const float* delta, int32_t n, int32_t count) {
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
@@ -215,6 +548,28 @@ __global__ void bc_check_sources_kernel(const int32_t* sources, int32_t nsrc, in
     if ((uint32_t)sources[i] >= (uint32_t)n) atomicCAS(status, 0u, (uint32_t)NPS_ERR_INVALID_ARG);
 }
 
+
+using BcKernel = void (*)(BcArgs);
+
+// The shared-memory kernel for n vertices, or null when they do not fit.  Threads per CTA
+// follow from how many CTAs an SM then holds: one fills it with 1,024, two or more take
+// 512 each, small graphs 256.
+BcKernel bc_pick_smem(size_t n, int device, int* threads) {
+  int limit = 0;
+  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return nullptr;
+  const size_t fixed = 2048;  // static shared memory
+  if (bc_smem_bytes(n, 1024) + fixed > (size_t)limit) return nullptr;
+  if (2 * (bc_smem_bytes(n, 512) + fixed) > (size_t)limit) {
+    *threads = 1024;
+    return bc_smem_kernel<1024>;
+  }
+  if (8 * (bc_smem_bytes(n, 256) + fixed) > (size_t)limit) {
+    *threads = 512;
+    return bc_smem_kernel<512>;
+  }
+  *threads = 256;
+  return bc_smem_kernel<256>;
+}
 
 struct BcWork {
   unsigned long long ctx_id = 0;  // context the cached buffers live in (nps_context_id)
@@ -312,9 +667,17 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   }
   // one CTA per source at a time, as many CTAs as are resident; a block of
   // sources shares one delta buffer
+  int threads = 0;  // of the shared-memory kernel; 0: the graph does not fit
+  const BcKernel smem_kernel = bc_pick_smem((size_t)n, p.device, &threads);
+  if (smem_kernel)
+    NPS_CUDA_RETURN(cudaFuncSetAttribute((const void*)smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)bc_smem_bytes((size_t)n, threads)));
+  const BcKernel kernel = smem_kernel ? smem_kernel : bc_sources_kernel;
+  const size_t dyn = smem_kernel ? bc_smem_bytes((size_t)n, threads) : 0;
+  if (!smem_kernel) threads = kThreads;
   int per_sm = 0;
-  NPS_CUDA_RETURN(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bc_sources_kernel, kThreads, 0));
-  const size_t per_cta = 4 * (size_t)n + 2;
+  NPS_CUDA_RETURN(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, threads, dyn));
+  const size_t per_cta = smem_kernel ? (size_t)n + 2 : 4 * (size_t)n + 2;
   // at most 8 GB of CTA scratch (16 n bytes each): large graphs run fewer sources at once
   const int64_t by_memory = std::max<int64_t>(W->sms, (int64_t)((8ull << 30) / (per_cta * sizeof(int32_t))));
   const int grid = (int)std::max<int64_t>(
@@ -338,14 +701,21 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   a.n = n;
   a.m = m;
   a.sources = dsrc;
-  a.level = W->scratch;
-  a.sigma = W->scratch + (size_t)n * grid;
-  a.order = W->scratch + 2 * (size_t)n * grid;
-  a.lb = W->scratch + 3 * (size_t)n * grid;
+  if (smem_kernel) {
+    a.level = a.sigma = a.order = nullptr;
+    a.lb = W->scratch;
+  } else {
+    a.level = W->scratch;
+    a.sigma = W->scratch + (size_t)n * grid;
+    a.order = W->scratch + 2 * (size_t)n * grid;
+    a.lb = W->scratch + 3 * (size_t)n * grid;
+  }
   a.delta = W->delta;
   a.status = W->status;
-  bc_fill_kernel<<<W->sms * 4, 256, 0, s>>>(a.level, a.sigma, (size_t)n * grid);
-  NPS_CUDA_RETURN(cudaGetLastError());
+  if (!smem_kernel) {
+    bc_fill_kernel<<<W->sms * 4, 256, 0, s>>>(a.level, a.sigma, (size_t)n * grid);
+    NPS_CUDA_RETURN(cudaGetLastError());
+  }
   uint32_t h_status = 0;
   if (dsrc && p.device_ptrs) {  // a bad device-side source list stops the call before any kernel reads it
     NPS_CUDA_RETURN(cudaMemcpyAsync(&h_status, W->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -357,7 +727,7 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   for (int32_t base = 0; base < count_all; base += block) {
     a.src_base = base;
     a.count = std::min<int32_t>(block, count_all - base);
-    bc_sources_kernel<<<grid, kThreads, 0, s>>>(a);
+    kernel<<<grid, threads, dyn, s>>>(a);
     NPS_CUDA_RETURN(cudaGetLastError());
     bc_fold_kernel<<<fold_grid, 256, 0, s>>>(dbc, W->delta, n, a.count);
     NPS_CUDA_RETURN(cudaGetLastError());
