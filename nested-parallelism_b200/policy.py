@@ -125,9 +125,7 @@ class GPUTrainer:
         if wt is not None:
             wt = t.as_tensor(wt, dtype=t.float32, device=self.dev).contiguous()
             wp = wt.data_ptr()
-        for g in self.grad:
-            g.zero_()
-        self.loss.zero_()
+        t._foreach_zero_([*self.grad, self.loss])  # one launch for the five
         check(lib.nps_mlp_loss_backward(self.w1_bf.data_ptr(), self.master[1].data_ptr(), self.w2_bf.data_ptr(),
                                         self.master[3].data_ptr(), X.data_ptr(), yd.data_ptr(), yl.data_ptr(),
                                         wp, X.shape[0], *[g.data_ptr() for g in self.grad],
