@@ -20,6 +20,9 @@
 //          described in a chunk table; a second kernel gives each chunk to a
 //          warp, and the warp that finishes a row's last chunk adds the row's
 //          chunk sums in chunk order
+// At the WARP and BLOCK levels, rows of at least kHubRow nonzeros take the GRID
+// level's chunks too: one warp or CTA walking a hub's row outlasts everything else.
+// R-MAT scale 20, threshold 64: WARP 2.15 -> 0.54 ms, BLOCK 1.16 -> 0.47 (GRID 0.19).
 //
 // Every y[r] is summed in an order fixed by the matrix alone (round by round,
 // then a fixed shuffle tree; chunk by chunk for GRID rows), so results repeat
@@ -47,6 +50,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kChunk = 1024;  // nonzeros per grid-level chunk
+// WARP and BLOCK levels: rows from kHubRow nonzeros on take grid-level chunks, in matrices of
+// at least kHubMinNnz (below, the second launch costs what a hub does: R-MAT 12 BLOCK 80 ->
+// 84 us, R-MAT 16 WARP 297 -> 163).
+constexpr int32_t kHubRow = 2048;
+constexpr int64_t kHubMinNnz = 1 << 19;
 constexpr int kStripes = 8;
 // Loads in flight per lane in a grid-level chunk, and the resident CTAs per SM
 // the chunk kernel is built for.  On R-MAT scale 22 the pairs (8, 4), (4, 5),
@@ -74,6 +82,13 @@ struct ChunkDesc {
   int32_t start;  // nonzero range [start, end)
   int32_t end;
   int32_t entry;  // list entry of the row when it has more than one chunk, else -1
+};
+
+// The lists of rows consolidated device-wide, and how many entries they hold.
+struct Lists {
+  LargeRow* row;
+  ChunkDesc* chunk;
+  uint32_t rows, chunks;
 };
 
 struct Mat {
@@ -210,6 +225,51 @@ __device__ __forceinline__ bool small_rows(const Mat& A, int64_t g, int32_t s, i
   return large;
 }
 
+// Lists the rows of group g whose lanes have `large` set, with their chunks.
+// Warp-collective.
+__device__ __forceinline__ void list_rows(bool large, int32_t deg, int32_t s, int32_t e, int64_t g,
+                                          const Lists& L, SpmvCtr* c, int lane) {
+  const unsigned lm = __ballot_sync(kFull, large);
+  if (!lm) return;
+  // one 64-bit atomic per warp reserves list entries and chunks together, so
+  // list order is chunk order
+  const uint32_t nch = large ? ((uint32_t)deg + kChunk - 1) / kChunk : 0u;
+  uint32_t cincl = nch;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, cincl, o);
+    if (lane >= o) cincl += t;
+  }
+  const uint32_t ctot = __shfl_sync(kFull, cincl, 31);
+  const int leader = __ffs(lm) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) base = atomicAdd(&c->list, ((unsigned long long)__popc(lm) << 32) | ctot);
+  base = __shfl_sync(kFull, base, leader);
+  const uint32_t slot = (uint32_t)(base >> 32) + __popc(lm & ((1u << lane) - 1));
+  const uint32_t cb = (uint32_t)base + (cincl - nch);
+  // valid rows fit; rows that overlap (malformed offsets) may not
+  const bool fits = !large || (slot < L.rows && (uint64_t)cb + nch <= L.chunks);
+  if (!__all_sync(kFull, fits)) {
+    flag_format(c);
+    return;
+  }
+  if (large && nch > 1) L.row[slot] = LargeRow{(int32_t)(g * 32 + lane), cb, nch, 0u};
+  // the chunk table, written by the whole warp one large row at a time
+  unsigned todo = lm;
+  while (todo) {
+    const int j = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const uint32_t js = __shfl_sync(kFull, slot, j), jcb = __shfl_sync(kFull, cb, j);
+    const uint32_t jn = __shfl_sync(kFull, nch, j);
+    const int32_t rs = __shfl_sync(kFull, s, j), re = __shfl_sync(kFull, e, j);
+    for (uint32_t i = lane; i < jn; i += 32) {
+      const int64_t cs = (int64_t)rs + (int64_t)i * kChunk;
+      L.chunk[jcb + i] = ChunkDesc{(int32_t)(g * 32 + j), (int32_t)cs, (int32_t)min((int64_t)re, cs + kChunk),
+                             jn > 1 ? (int32_t)js : -1};
+    }
+  }
+}
+
 // Next row group for a warp from kStripes striped counters: one atomic, issued
 // by lane 0, whose result is used one group later so its latency overlaps the
 // walk.  A stripe that runs dry sends the warp to the next stripe.
@@ -244,9 +304,8 @@ struct GroupFeed {
 // WARP and GRID levels: warps take row groups on their own.  The group after
 // the current one is known and its row bounds are loading while the current
 // group is walked, and the ticket for the one after that is in flight.
-template <int LEVEL>
-__global__ void __launch_bounds__(kThreads) spmv_rows_kernel(Mat A, int32_t threshold, LargeRow* L, ChunkDesc* D,
-                                                             SpmvCtr* c) {
+template <int LEVEL, bool HUBS>
+__global__ void __launch_bounds__(kThreads) spmv_rows_kernel(Mat A, int32_t threshold, Lists L, SpmvCtr* c) {
   const int lane = threadIdx.x & 31;
   const int gw = blockIdx.x * kWarps + (threadIdx.x >> 5);
   GroupFeed f;
@@ -265,7 +324,9 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_kernel(Mat A, int32_t thre
     const bool large = small_rows(A, g, s, e, threshold, lane, c);
     const int32_t deg = e - s;
     if (LEVEL == NPS_LEVEL_WARP) {
-      unsigned lm = __ballot_sync(kFull, large);
+      const bool hub = HUBS && large && deg >= kHubRow;
+      if (HUBS) list_rows(hub, deg, s, e, g, L, c, lane);
+      unsigned lm = __ballot_sync(kFull, large && !hub);
       while (lm) {
         const int j = __ffs(lm) - 1;
         lm &= lm - 1;
@@ -274,40 +335,7 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_kernel(Mat A, int32_t thre
         if (lane == 0) A.y[g * 32 + j] = t;
       }
     } else {
-      // one 64-bit atomic per warp reserves list entries and chunks together, so
-      // list order is chunk order
-      const uint32_t nch = large ? ((uint32_t)deg + kChunk - 1) / kChunk : 0u;
-      const unsigned lm = __ballot_sync(kFull, large);
-      if (lm) {
-        uint32_t cincl = nch;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(kFull, cincl, o);
-          if (lane >= o) cincl += t;
-        }
-        const uint32_t ctot = __shfl_sync(kFull, cincl, 31);
-        const int leader = __ffs(lm) - 1;
-        unsigned long long base = 0;
-        if (lane == leader) base = atomicAdd(&c->list, ((unsigned long long)__popc(lm) << 32) | ctot);
-        base = __shfl_sync(kFull, base, leader);
-        const uint32_t slot = (uint32_t)(base >> 32) + __popc(lm & ((1u << lane) - 1));
-        const uint32_t cb = (uint32_t)base + (cincl - nch);
-        if (large && nch > 1) L[slot] = LargeRow{(int32_t)(g * 32 + lane), cb, nch, 0u};
-        // the chunk table, written by the whole warp one large row at a time
-        unsigned todo = lm;
-        while (todo) {
-          const int j = __ffs(todo) - 1;
-          todo &= todo - 1;
-          const uint32_t js = __shfl_sync(kFull, slot, j), jcb = __shfl_sync(kFull, cb, j);
-          const uint32_t jn = __shfl_sync(kFull, nch, j);
-          const int32_t rs = __shfl_sync(kFull, s, j), re = __shfl_sync(kFull, e, j);
-          for (uint32_t i = lane; i < jn; i += 32) {
-            const int64_t cs = (int64_t)rs + (int64_t)i * kChunk;
-            D[jcb + i] = ChunkDesc{(int32_t)(g * 32 + j), (int32_t)cs, (int32_t)min((int64_t)re, cs + kChunk),
-                                   jn > 1 ? (int32_t)js : -1};
-          }
-        }
-      }
+      list_rows(large, deg, s, e, g, L, c, lane);
     }
     g = gn;
     s = sn;
@@ -320,7 +348,7 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_kernel(Mat A, int32_t thre
 // kStripes striped counters); each CTA lists its large rows in shared memory and
 // walks each with all its threads.  The unit loop is the same for every thread
 // of the CTA, so its barriers are reached by all.
-__global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_t threshold, SpmvCtr* c) {
+__global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_t threshold, Lists L, SpmvCtr* c) {
   __shared__ int32_t s_rows[kThreads];
   __shared__ uint32_t s_count[2];  // per unit parity, like s_unit: reset two units after its last read
   __shared__ double s_part[kWarps];
@@ -354,7 +382,9 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_
       const int64_t r = g * 32 + lane;
       int32_t s = 0, e = 0;
       if (r < A.n) row_bounds(A, r, s, e, c);
-      if (small_rows(A, g, s, e, threshold, lane, c)) s_rows[atomicAdd(&s_count[it & 1], 1u)] = (int32_t)r;
+      const bool large = small_rows(A, g, s, e, threshold, lane, c), hub = large && e - s >= kHubRow && L.rows;
+      list_rows(hub, e - s, s, e, g, L, c, lane);
+      if (large && !hub) s_rows[atomicAdd(&s_count[it & 1], 1u)] = (int32_t)r;
     }
     __syncthreads();
     const uint32_t cnt = s_count[it & 1];
@@ -389,24 +419,26 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_
 // chunk's descriptor loading while the current one is walked.  A row of one
 // chunk is written at once; for longer rows the warp that finishes the last
 // chunk adds the row's chunk sums in chunk order.
-__global__ void __launch_bounds__(kThreads, kChunkCtas) spmv_chunks_kernel(Mat A, LargeRow* L, const ChunkDesc* D, double* part,
+__global__ void __launch_bounds__(kThreads, kChunkCtas) spmv_chunks_kernel(Mat A, Lists L, double* part,
                                                                SpmvCtr* c) {
-  const uint32_t nc = (uint32_t)c->list;
+  cudaGridDependencySynchronize();  // launched ahead of the row pass's end, which it waits for here
+  if (c->status) return;            // the lists may have holes
+  const uint32_t nc = min((uint32_t)c->list, L.chunks);
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * kWarps;
   uint32_t q = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  ChunkDesc cd = q < nc ? D[q] : ChunkDesc{0, 0, 0, -1};
+  ChunkDesc cd = q < nc ? L.chunk[q] : ChunkDesc{0, 0, 0, -1};
   for (; q < nc; q += warps) {
-    const ChunkDesc nx = q + warps < nc ? D[q + warps] : ChunkDesc{0, 0, 0, -1};
+    const ChunkDesc nx = q + warps < nc ? L.chunk[q + warps] : ChunkDesc{0, 0, 0, -1};
     const double t = warp_range<kBatch>(A, cd.start, cd.end, lane, c);
     if (lane == 0) {
       if (cd.entry < 0) {
         A.y[cd.row] = t;
       } else {
-        const LargeRow lr = L[cd.entry];
+        const LargeRow lr = L.row[cd.entry];
         part[q] = t;
         __threadfence();
-        if (atomicAdd(&L[cd.entry].done, 1u) == lr.chunks - 1) {  // the row's last chunk
+        if (atomicAdd(&L.row[cd.entry].done, 1u) == lr.chunks - 1) {  // the row's last chunk
           __threadfence();
           double sum = 0.0;
           for (uint32_t i = 0; i < lr.chunks; ++i) sum += __ldcg(part + lr.chunk_begin + i);
@@ -519,32 +551,45 @@ extern "C" nps_status nps_spmv(const int32_t* row_ptr, const int32_t* col, const
   }
   const int grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(((int64_t)n + kThreads - 1) / kThreads, (int64_t)W->sms * (2048 / kThreads)));
-  LargeRow* L = nullptr;
-  ChunkDesc* D = nullptr;
-  if (p.level == NPS_LEVEL_GRID) {
-    // large rows <= m / threshold; chunks <= m / kChunk + large rows
-    const size_t nl = std::min<size_t>((size_t)n, (size_t)m / (size_t)p.threshold + 1);
+  Lists L{nullptr, nullptr, 0, 0};
+  // shortest row that goes to the list; none does without one
+  const int32_t list_from = p.level == NPS_LEVEL_GRID ? p.threshold : std::max(p.threshold, kHubRow);
+  const bool lists = m >= (p.level == NPS_LEVEL_GRID ? (int64_t)list_from : kHubMinNnz);
+  if (lists) {
+    // listed rows <= m / list_from; chunks <= m / kChunk + listed rows
+    const size_t nl = std::min<size_t>((size_t)n, (size_t)m / (size_t)list_from + 1);
     const size_t nc = (size_t)m / kChunk + nl + 1;
     if ((e = nps_ensure(&W->list, &W->list_n, nl, s, "spmv")) || (e = nps_ensure(&W->part, &W->part_n, nc, s, "spmv")) ||
         (e = nps_ensure(&W->chunks, &W->chunks_n, nc, s, "spmv")))
       return e;
-    L = W->list;
-    D = W->chunks;
+    L = Lists{W->list, W->chunks, (uint32_t)nl, (uint32_t)nc};
   }
   NPS_CUDA_RETURN(cudaMemsetAsync(W->ctr, 0, sizeof(SpmvCtr), s));
   NPS_CUDA_RETURN(cudaEventRecord(W->ev[1], s));
   switch (p.level) {
     case NPS_LEVEL_WARP:
-      spmv_rows_kernel<NPS_LEVEL_WARP><<<grid, kThreads, 0, s>>>(A, p.threshold, L, D, W->ctr);
+      if (lists) spmv_rows_kernel<NPS_LEVEL_WARP, true><<<grid, kThreads, 0, s>>>(A, p.threshold, L, W->ctr);
+      else spmv_rows_kernel<NPS_LEVEL_WARP, false><<<grid, kThreads, 0, s>>>(A, p.threshold, L, W->ctr);
       break;
     case NPS_LEVEL_BLOCK:
-      spmv_rows_block_kernel<<<grid, kThreads, 0, s>>>(A, p.threshold, W->ctr);
+      spmv_rows_block_kernel<<<grid, kThreads, 0, s>>>(A, p.threshold, L, W->ctr);
       break;
     default:
-      spmv_rows_kernel<NPS_LEVEL_GRID><<<grid, kThreads, 0, s>>>(A, p.threshold, L, D, W->ctr);
-      NPS_CUDA_RETURN(cudaGetLastError());
-      spmv_chunks_kernel<<<grid, kThreads, 0, s>>>(A, L, D, W->part, W->ctr);
+      spmv_rows_kernel<NPS_LEVEL_GRID, true><<<grid, kThreads, 0, s>>>(A, p.threshold, L, W->ctr);
       break;
+  }
+  NPS_CUDA_RETURN(cudaGetLastError());
+  if (lists) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    NPS_CUDA_RETURN(cudaLaunchKernelEx(&cfg, spmv_chunks_kernel, A, L, W->part, W->ctr));
   }
   NPS_CUDA_RETURN(cudaGetLastError());
   NPS_CUDA_RETURN(cudaEventRecord(W->ev[2], s));
@@ -557,7 +602,8 @@ extern "C" nps_status nps_spmv(const int32_t* row_ptr, const int32_t* col, const
     st->grid_ctas = grid;
     st->edges_scanned = (uint64_t)m;
     st->vertices_processed = (uint64_t)n;
-    st->buckets = (uint32_t)(W->h_ctr->list >> 32);  // grid level: rows consolidated device-wide
+    if (p.level == NPS_LEVEL_GRID)
+      st->buckets = (uint32_t)(W->h_ctr->list >> 32);  // rows consolidated device-wide
     cudaEventElapsedTime(&st->kernel_ms, W->ev[1], W->ev[2]);
     cudaEventElapsedTime(&st->total_ms, W->ev[0], W->ev[3]);
   }
