@@ -78,8 +78,17 @@ constexpr int kBlockListCap = 512;     // CTA list entries (block tier)
 constexpr int kHopCap = 256;
 constexpr int kHopStop = 128;
 constexpr uint32_t kHopSeeds = 32;
+// ... and their edges, at the graph's average degree: more give the item loop enough, and
+// there the distance check before the atomicMin pays.  Uniform 18,604 x 202,728, unordered,
+// at 64 / 128 / 192 edges and without this limit: 0.152 / 0.148 / 0.160 / 0.184 ms.
+constexpr uint32_t kHopSeedEdges = 128;
 constexpr uint32_t kHopMinSeeds = 2;
 constexpr int kHopRounds = 32;
+// Rounds that list rows are a sign of a power-law frontier: its long rows wait an iteration
+// and the short ones run ahead of them, with distances that the long rows lower again.
+// Rounds then pause for kHopPause iterations, twice as many each time.  R-MAT 15, edge
+// factor 8, block level, unordered: 0.23 ms a call without rounds, 0.32 without the pause.
+constexpr uint32_t kHopPause = 8;
 constexpr int32_t kHopList = 128;
 
 // Per-instance device counters.  Zeroed by the host before a launch.
@@ -903,6 +912,9 @@ struct Smem {
                                  // this round and the next
   };
   HopArgs hop_args;            // CTA rounds: the iteration, written by thread 0
+  uint32_t hop_seeds;          // CTA rounds: frontier vertices per CTA up to which they run
+  uint32_t hop_it, hop_from, hop_pause;  // CTA rounds: last iteration of rounds; the first one they
+                               // may run in next; how long they pause when rows were listed
   uint32_t hop_n[3];           // CTA rounds: entries pushed for round r in hop_n[r % 3]
   unsigned long long hop_acc[4];         // CTA rounds: edges, improvements, first reaches, vertices of the solve
   int32_t stage[BS / 32][3][kStage];  // per-warp append staging: [near, far, settle]
@@ -1852,6 +1864,13 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
   // ---- prologue: distances, stamps, initial frontier, first bucket
   uint32_t base = 0, qlen = 0, delta = 0;
   int level = 0;
+  if (threadIdx.x == 0) {
+    sm.hop_it = 0xffffffffu;
+    sm.hop_from = 0;
+    sm.hop_pause = kHopPause;
+    sm.hop_seeds = max(1u, min(kHopSeeds, (uint32_t)((unsigned long long)kHopSeedEdges * (uint32_t)I.n /
+                                                     (uint32_t)max(I.m, 1))));
+  }
   if (!start_instance<BS>(P, I, sm, bar, bar_epoch, rank, team_size, inject, learned, base, qlen, delta, level))
     return;
   uint32_t it = 0, ep = 0;
@@ -1940,8 +1959,9 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     // the far pile and the settle list, nor where a pass per frontier is asked for: the
     // policy's and the trace's per-iteration statistics, degree ordering, local rounds.
     const bool hops = !advance && !heavy_it && !want_iter && hprev_tot == 0 && C.local_rounds == 0 &&
-                      C.order_deg == 0 && qlen <= team_size * kHopSeeds;
+                      C.order_deg == 0 && qlen <= team_size * sm.hop_seeds && it >= sm.hop_from;
     if (hops && threadIdx.x == 0) {
+      sm.hop_it = it;
       const uint32_t per = max(kHopMinSeeds, (qlen + team_size - 1) / team_size);
       sm.hop_args.srcq = I.q[it & 1];
       sm.hop_args.begin = min(qlen, rank * per);
@@ -2133,6 +2153,10 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       sm.bc_m = m1;
       sm.bc_s = s1;
       sm.bc_ag = ag;
+      if (sm.hop_it == it && h1 != 0) {  // CTA rounds listed rows (every CTA read the same count)
+        sm.hop_from = it + 1 + sm.hop_pause;
+        sm.hop_pause *= 2;
+      }
       if (st1 != 0) {
         atomicExch(P.abort_flag, 1u);
         sm.ok = 0;

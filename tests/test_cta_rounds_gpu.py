@@ -128,3 +128,23 @@ def test_malformed_rows_and_heads_are_reported(nps, cuda_device):
         with pytest.raises(nps.NpsError) as ei:
             nps.sssp_device(*t, g.n, g.m, 0, out, nps.Params(level=2))
         assert ei.value.status == 7
+
+
+@pytest.mark.parametrize("ef", [2, 8, 24])
+@pytest.mark.parametrize("level", [0, 1, 2])
+def test_rounds_pause_where_rows_are_listed(nps, oracle, cuda_device, ef, level):
+    """Long rows met in rounds (power-law graphs, from a hub and from a leaf) and a road
+    with hubs, so that rounds run, pause and run again; average degrees from 2 to 24 move
+    the seed limit."""
+    g = nps.gen_rmat(12, ef, seed=ef)
+    leaf = int(np.flatnonzero((g.degrees() > 0) & (g.degrees() < 4))[0])
+    n = 4000
+    hubs = np.arange(0, n, 500)
+    s = np.concatenate([np.arange(n - 1), np.repeat(hubs, 200)])
+    d = np.concatenate([np.arange(1, n), (np.repeat(hubs, 200) + np.tile(np.arange(200), hubs.size) * 7 + 2) % n])
+    road = nps.convertCSR(n, s, d, (np.arange(s.size) % 90 + 1).astype(np.uint32))
+    for delta in (0, 64):
+        p = nps.Params(level=level, threshold=32, delta=delta)
+        _check(nps, oracle, g, p, g.source)
+        _check(nps, oracle, g, p, leaf)
+        _check(nps, oracle, road, p)
