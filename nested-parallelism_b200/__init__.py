@@ -228,8 +228,7 @@ class Params:
     sort_at_push: int = 0               # grid-tier rows sorted at push: 1 on, -1 off, 0 by the grid threshold
 
     def to_c(self, device_ptrs: bool, stream: Optional[int] = None) -> nps_params:
-        p = nps_params()
-        lib.nps_params_default(C.byref(p))
+        p = nps_params()  # zeroed; every other field is set below
         p.level, p.threshold = self.level, self.threshold
         p.block_threshold, p.grid_threshold = self.block_threshold, self.grid_threshold
         p.block_size, p.ctas_per_sm, p.delta = self.block_size, self.ctas_per_sm, self.delta

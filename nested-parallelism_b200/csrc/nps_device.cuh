@@ -206,7 +206,7 @@ struct PolicyDev {
 struct LaunchParams {
   InstDesc* inst;
   const int32_t* order;
-  const TeamDesc* teams;
+  const TeamDesc* teams;  // batches
   int32_t n_teams;
   int32_t fault_inject_wait;  // 1: the first barrier waits for an arrival that never comes
   int32_t test_disagree;      // 1: CTA 1 reports another hash for the first decision (agreement check test)
@@ -2695,13 +2695,17 @@ __global__ void __launch_bounds__(BS, kMinBlocks<BS>) sssp_persistent_kernel(con
   __shared__ InstDesc sinst;
   if (threadIdx.x == 0) {
     sm.t_start = globaltimer_ns();
-    sm.team_id = -1;
-    for (int t = 0; t < P.n_teams; ++t) {
-      TeamDesc td = P.teams[t];
+    sm.team_id = SINGLE ? 0 : -1;
+    if (SINGLE) sm.team = TeamDesc{0, (int32_t)gridDim.x, 0, 1};  // one team: every CTA
+  }
+  if constexpr (!SINGLE) {
+    // the team whose CTA range holds this one: the table read side by side
+    __syncthreads();
+    for (int t = threadIdx.x; t < P.n_teams; t += BS) {
+      const TeamDesc td = P.teams[t];
       if ((int)blockIdx.x >= td.cta_begin && (int)blockIdx.x < td.cta_begin + td.cta_count) {
         sm.team = td;
         sm.team_id = t;
-        break;
       }
     }
   }

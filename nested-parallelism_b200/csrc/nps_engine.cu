@@ -14,10 +14,11 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <cstddef>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <queue>
-#include <set>
 #include <string>
 #include <vector>
 
@@ -170,13 +171,9 @@ KernelFn pick_kernel(int bs, bool single, bool async, bool lean) {
 // Shared-memory carveout: the smallest split that still holds `nb` resident
 // CTAs, so the rest of the SM's 256 KB of L1/shared storage caches the
 // distance array (the pre-check loads of hub vertices hit in L1 instead of
-// queueing on one L2 slice).  Done once per (device, kernel); occupancy is
-// checked again and the default restored if the split would lower it.
+// queueing on one L2 slice).  Occupancy is checked again and the default
+// restored if the split would lower it.
 cudaError_t set_carveout(int dev, KernelFn k, int bs, int nb) {
-  static std::mutex mu;
-  static std::set<std::pair<int, const void*>> done;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!done.insert({dev, (const void*)k}).second) return cudaSuccess;
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)k);
   if (e != cudaSuccess) return e;
@@ -195,17 +192,28 @@ cudaError_t set_carveout(int dev, KernelFn k, int bs, int nb) {
   return cudaSuccess;
 }
 
+// Grid of the persistent kernel: its resident CTAs per SM, asked for (and the carveout
+// set) once per device and kernel.
 nps_status grid_size(int dev, const DevInfo& di, int bs, bool single, int ctas_per_sm, int* grid,
                      bool async, bool lean) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, int> resident;
   KernelFn k = pick_kernel(bs, single, async, lean);
   if (!k) return nps_fail(NPS_ERR_INVALID_ARG, "block_size must be 128, 256 or 512");
   int nb = 0;
-  NPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void*)k, bs, 0));
-  if (nb <= 0) return nps_fail(NPS_ERR_CUDA, "persistent kernel does not fit on an SM");
-  NPS_CUDA(set_carveout(dev, k, bs, nb));
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    int& known = resident[{dev, (const void*)k}];
+    if (known == 0) {
+      NPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void*)k, bs, 0));
+      if (nb <= 0) return nps_fail(NPS_ERR_CUDA, "persistent kernel does not fit on an SM");
+      NPS_CUDA(set_carveout(dev, k, bs, nb));
+      known = nb;
+    }
+    nb = known;
+  }
   if (ctas_per_sm > 0) nb = std::min(nb, ctas_per_sm);
   *grid = nb * di.sms;
-  (void)dev;
   return NPS_OK;
 }
 
@@ -243,7 +251,7 @@ struct DevBuf {
 
 // Control block: counters, barrier words and the abort flag share one
 // allocation so a single memset clears them before each launch.  Layout:
-//   Counters[n_inst] | barrier words, `stride` per team | abort flag (128 B) | team table (128 B)
+//   Counters[n_inst] | barrier words, `stride` per team | abort flag (128 B)
 struct Control {
   size_t n_inst = 0, n_teams = 0, stride = 0;
   char* base = nullptr;
@@ -254,9 +262,7 @@ struct Control {
   Counters* ctr() const { return (Counters*)base; }
   uint32_t* bar() const { return (uint32_t*)(base + counters_bytes()); }
   uint32_t* abort_flag() const { return (uint32_t*)(base + counters_bytes() + bar_bytes()); }
-  TeamDesc* team_table() const { return (TeamDesc*)(base + counters_bytes() + bar_bytes() + 128); }
-  size_t clear_bytes() const { return counters_bytes() + bar_bytes() + 128; }
-  size_t bytes() const { return clear_bytes() + 128; }
+  size_t bytes() const { return counters_bytes() + bar_bytes() + 128; }
 };
 
 struct PolicyState {
@@ -307,6 +313,7 @@ struct nps_ctx {
   nps_params b_params_key{};
   int b_grid = 0, b_bs = 0;
   int b_nteams = 0;
+  bool b_built = false;  // the buffers describe b_key's set
   cudaGraphExec_t b_graph = nullptr;
   // Re-balancing of the teams of an unchanged instance set (one instance per team):
   // stage 0 splits CTAs by work; the solve times of the first two calls (taken with
@@ -630,9 +637,6 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
     d.wait_ns = (unsigned long long)(p.timeout_s * 1e9);
   }
 
-  TeamDesc td{0, grid, 0, 1};
-  // single-instance launches read the team table from a small device buffer
-  static_assert(sizeof(TeamDesc) == 16, "team descriptor layout");
   LaunchParams lp;
   memset(&lp, 0, sizeof(lp));
   lp.inst = nullptr;
@@ -648,15 +652,12 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   lp.policy = policy_ptr(c->device);
   if (p.policy == NPS_POLICY_LEARNED && !lp.policy)
     return nps_fail(NPS_ERR_INVALID_ARG, "learned policy requested but no weights loaded (nps_policy_set_weights)");
-  TeamDesc* d_team = ctl.team_table();
-  lp.teams = d_team;
-
-  NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s));
-  NPS_CUDA(cudaMemcpyAsync(d_team, &td, sizeof(td), cudaMemcpyHostToDevice, s));
+  NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.bytes(), s));
   if (time_it) NPS_CUDA(cudaEventRecord(c->ev[1], s));
   if ((e = launch(c, s, p.block_size, true, nps_lean(p), grid, lp, d))) return e;
   if (time_it) NPS_CUDA(cudaEventRecord(c->ev[2], s));
-  NPS_CUDA(cudaMemcpyAsync(c->h_ctr, ctl.ctr(), sizeof(Counters), cudaMemcpyDeviceToHost, s));
+  // the work counters at the struct's end stay on the device
+  NPS_CUDA(cudaMemcpyAsync(c->h_ctr, ctl.ctr(), offsetof(Counters, work), cudaMemcpyDeviceToHost, s));
   if (st) st->grid_ctas = grid;
   return NPS_OK;
 }
@@ -973,15 +974,18 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
                         memcmp(&c->b_params_key, &p, sizeof(p)) == 0;
   const int nteams = std::min(count, grid);
   if (!same_set || nteams != count) c->b_stage = 0;
-  // stages 1 and 2 form the teams anew (a captured graph is captured again); stage 3
-  // keeps the last split
+  // stages 1 and 2 form the teams anew; stage 3 keeps the last split.  Calls that form
+  // teams launch directly: a graph pays for its capture and instantiation (about 0.2 ms
+  // for 64 instances) only when the launch is repeated as it is, so it is captured by the
+  // first call that repeats one.
   const bool rebalance = c->b_stage == 1 || c->b_stage == 2;
-  const bool same = same_set && c->b_graph && !rebalance;
+  const bool same = same_set && c->b_built && !rebalance;
   Control ctl((size_t)count, (size_t)nteams, grid);
 
   if (!same) {
     if (c->b_graph) cudaGraphExecDestroy(c->b_graph);
     c->b_graph = nullptr;
+    c->b_built = false;
     // workspace: per instance 4 queues of n int32 + marks carved from pools
     size_t q_total = 0, h_total = 0;
     std::vector<uint32_t> hcap(count), icap(count), ishift(count);
@@ -1117,7 +1121,8 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
     NPS_CUDA(cudaMemcpyAsync(c->b_inst.p, c->b_inst_host.data(), sizeof(InstDesc) * count, cudaMemcpyHostToDevice, s));
     NPS_CUDA(cudaMemcpyAsync(c->b_teams.p, teams.data(), sizeof(TeamDesc) * nteams, cudaMemcpyHostToDevice, s));
     NPS_CUDA(cudaMemcpyAsync(c->b_order.p, order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, s));
-    NPS_CUDA(cudaStreamSynchronize(s));  // host vectors above go out of scope
+    // (pageable sources: each copy has left the host vectors when its call returns)
+    c->b_built = true;
     c->b_key.assign(inst, inst + count);
     c->b_params_key = p;
     c->b_grid = grid;
@@ -1146,11 +1151,11 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
   if ((e = ensure_pinned_counters(c, (size_t)count))) return e;
 
   NPS_CUDA(cudaEventRecord(c->ev[1], s));
-  if (use_graph) {
+  if (use_graph && same) {
     if (!c->b_graph) {
       cudaGraph_t g = nullptr;
       NPS_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      cudaError_t ce = cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s);
+      cudaError_t ce = cudaMemsetAsync(ctl.base, 0, ctl.bytes(), s);
       nps_status le = ce == cudaSuccess ? launch(c, s, p.block_size, false, nps_lean(p), grid, lp, dummy) : NPS_ERR_CUDA;
       cudaError_t ee = cudaStreamEndCapture(s, &g);
       if (ce != cudaSuccess) return nps_fail(NPS_ERR_CUDA, std::string("capture memset: ") + cudaGetErrorString(ce));
@@ -1169,7 +1174,7 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
     }
     NPS_CUDA(cudaGraphLaunch(c->b_graph, s));
   } else {
-    NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.clear_bytes(), s));
+    NPS_CUDA(cudaMemsetAsync(ctl.base, 0, ctl.bytes(), s));
     if ((e = launch(c, s, p.block_size, false, nps_lean(p), grid, lp, dummy))) return e;
   }
   NPS_CUDA(cudaEventRecord(c->ev[2], s));

@@ -46,7 +46,6 @@ namespace {
 using nps::Counters;
 using nps::InstDesc;
 using nps::LaunchParams;
-using nps::TeamDesc;
 
 constexpr size_t kMaxV = NPS_NOALLOC_MAX_VERTICES;
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -56,9 +55,8 @@ constexpr size_t kBarWords = 4096;  // one team of up to 2032 CTAs (2 + 2032/16 
 constexpr size_t kOffCtr = 0;
 constexpr size_t kOffBar = align256(kOffCtr + sizeof(Counters));
 constexpr size_t kOffAbort = align256(kOffBar + kBarWords * sizeof(uint32_t));
-constexpr size_t kOffTeam = align256(kOffAbort + 128);
-constexpr size_t kClearBytes = kOffTeam;  // counters, barrier words, abort flag
-constexpr size_t kOffStamp = align256(kOffTeam + sizeof(TeamDesc));
+constexpr size_t kOffStamp = align256(kOffAbort + 128);
+constexpr size_t kClearBytes = kOffStamp;  // counters, barrier words, abort flag
 constexpr size_t kOffMarks = align256(kOffStamp + sizeof(uint32_t));
 constexpr size_t kOffQueues = align256(kOffMarks + 3 * kMaxV * sizeof(uint32_t));
 constexpr size_t kOffHeavy = align256(kOffQueues + 6 * kMaxV * sizeof(int32_t));
@@ -225,10 +223,8 @@ extern "C" nps_status nps_sssp_noalloc(const int32_t* d_row_ptr, const int32_t* 
   d.dsched = p.delta_schedule;
   d.sort_push = p.sort_at_push < -1 ? -1 : (p.sort_at_push > 1 ? 1 : p.sort_at_push);
 
-  const TeamDesc td{0, grid, 0, 1};
   LaunchParams lp;
   memset(&lp, 0, sizeof(lp));
-  lp.teams = (const TeamDesc*)(base + kOffTeam);
   lp.n_teams = 1;
   lp.fault_inject_wait = p.reserved[0] == 1;
   lp.test_disagree = p.reserved[0] == 2;
@@ -241,7 +237,6 @@ extern "C" nps_status nps_sssp_noalloc(const int32_t* d_row_ptr, const int32_t* 
 
   // counters, barrier words and the abort flag start at zero on every call
   NA_CUDA(cudaMemsetAsync(base + kOffCtr, 0, kClearBytes, s));
-  NA_CUDA(cudaMemcpyAsync(base + kOffTeam, &td, sizeof(td), cudaMemcpyHostToDevice, s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)p.block_size);
