@@ -300,6 +300,8 @@ struct nps_ctx {
   DevBuf<uint8_t> g_wpack;     // weights packed to 1 or 2 bytes, widened into g_w
   uint8_t* h_wpack = nullptr;  // pinned staging of the packed weights
   size_t h_wpack_n = 0;
+  uint8_t* h_stage = nullptr;  // pinned slots for copies from pageable host arrays (kStageSlots of kStageBytes)
+  cudaEvent_t stage_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // the last copy out of each slot
   // batch workspace
   DevBuf<int32_t> b_pool;
   DevBuf<uint32_t> b_stamp;
@@ -364,6 +366,10 @@ void ctx_release(nps_ctx* c) {
   if (c->h_wpack) cudaFreeHost(c->h_wpack);
   c->h_wpack = nullptr;
   c->h_wpack_n = 0;
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  c->h_stage = nullptr;
+  for (auto& e : c->stage_ev)
+    if (e) cudaEventDestroy(e);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -779,6 +785,94 @@ nps_status ensure_pinned_wpack(nps_ctx* c, size_t bytes) {
   return NPS_OK;
 }
 
+// Host-to-device copy of a graph array.  The driver moves pageable memory through its own
+// staging with one thread, about 10 GB/s; here the host's threads fill pinned slots that
+// the copy engine empties behind them.  Pinned arrays, arrays below kStageMin and a host
+// without room for the slots take the plain copy.  A call on pageable arrays, 16 cores:
+// R-MAT 18 2.0 -> 1.2 ms, R-MAT 20 8.8 -> 4.2 ms.
+constexpr size_t kStageBytes = (size_t)2 << 20;
+constexpr int kStageSlots = 4;
+constexpr size_t kStageMin = (size_t)1 << 20;
+
+bool stage_ready(nps_ctx* c) {
+  if (c->h_stage) return true;
+  for (auto& e : c->stage_ev)
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  if (cudaMallocHost(&c->h_stage, kStageSlots * kStageBytes) != cudaSuccess) {
+    cudaGetLastError();
+    c->h_stage = nullptr;
+    return false;
+  }
+  return true;
+}
+
+// Whether a copy of `bytes` from or to host memory at p goes through the slots.
+bool staged(nps_ctx* c, const void* p, size_t bytes) {
+  if (bytes < kStageMin) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered && stage_ready(c);
+}
+
+// memcpy by the host's threads.
+void copy_pieces(uint8_t* dst, const uint8_t* src, size_t n) {
+  constexpr size_t kPiece = (size_t)64 << 10;
+  const int64_t pieces = (int64_t)((n + kPiece - 1) / kPiece);
+#pragma omp parallel for schedule(static)
+  for (int64_t k = 0; k < pieces; ++k)
+    memcpy(dst + (size_t)k * kPiece, src + (size_t)k * kPiece, std::min(kPiece, n - (size_t)k * kPiece));
+}
+
+nps_status copy_in(nps_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (!staged(c, src, bytes)) {
+    NPS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+    return NPS_OK;
+  }
+  size_t i = 0;
+  for (size_t off = 0; off < bytes; off += kStageBytes, ++i) {
+    const size_t n = std::min(kStageBytes, bytes - off);
+    const int slot = (int)(i % kStageSlots);
+    uint8_t* const h = c->h_stage + (size_t)slot * kStageBytes;
+    NPS_CUDA(cudaEventSynchronize(c->stage_ev[slot]));  // done at once for a slot not yet used
+    copy_pieces(h, static_cast<const uint8_t*>(src) + off, n);
+    NPS_CUDA(cudaMemcpyAsync(static_cast<uint8_t*>(dst) + off, h, n, cudaMemcpyHostToDevice, s));
+    NPS_CUDA(cudaEventRecord(c->stage_ev[slot], s));
+  }
+  return NPS_OK;
+}
+
+// Device-to-host copy of a result, behind the work queued on s.  Through the slots it has
+// ended when this returns, else it is queued.
+nps_status copy_out(nps_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (!staged(c, dst, bytes)) {
+    NPS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+    return NPS_OK;
+  }
+  const size_t chunks = (bytes + kStageBytes - 1) / kStageBytes;
+  for (size_t i = 0; i < chunks + kStageSlots; ++i) {
+    if (i >= kStageSlots) {  // chunk i - kStageSlots to its place
+      const size_t j = i - kStageSlots, off = j * kStageBytes;
+      NPS_CUDA(cudaEventSynchronize(c->stage_ev[j % kStageSlots]));
+      copy_pieces(static_cast<uint8_t*>(dst) + off, c->h_stage + (j % kStageSlots) * kStageBytes,
+                  std::min(kStageBytes, bytes - off));
+      if (j + 1 == chunks) break;
+    }
+    if (i < chunks) {
+      const size_t off = i * kStageBytes;
+      NPS_CUDA(cudaMemcpyAsync(c->h_stage + (i % kStageSlots) * kStageBytes, static_cast<const uint8_t*>(src) + off,
+                               std::min(kStageBytes, bytes - off), cudaMemcpyDeviceToHost, s));
+      NPS_CUDA(cudaEventRecord(c->stage_ev[i % kStageSlots], s));
+    }
+  }
+  return NPS_OK;
+}
+
 // nps_sssp_ctx, and with bfs = true nps_bfs (w unused: every edge weighs 1).
 nps_status sssp_ctx_impl(nps_ctx* c, const int32_t* row_ptr, const int32_t* col, const uint32_t* w, int32_t n,
                          int64_t m, int32_t src, const nps_params* pin, uint32_t* dist_out, nps_stats* st,
@@ -811,9 +905,9 @@ nps_status sssp_ctx_impl(nps_ctx* c, const int32_t* row_ptr, const int32_t* col,
     if ((e = c->g_row.ensure((size_t)n + 1, false, s)) || (e = c->g_col.ensure((size_t)m, false, s)) ||
         (!bfs && (e = c->g_w.ensure((size_t)m, false, s))) || (e = c->g_dist.ensure((size_t)n, false, s)))
       return e;
-    NPS_CUDA(cudaMemcpyAsync(c->g_row.p, row_ptr, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, s));
+    if ((e = copy_in(c, c->g_row.p, row_ptr, sizeof(int32_t) * ((size_t)n + 1), s))) return e;
     if (m > 0) {
-      NPS_CUDA(cudaMemcpyAsync(c->g_col.p, col, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
+      if ((e = copy_in(c, c->g_col.p, col, sizeof(int32_t) * (size_t)m, s))) return e;
       if (!bfs) {
         int wb = 4;
         if (m >= kPackMinEdges) {
@@ -826,7 +920,7 @@ nps_status sssp_ctx_impl(nps_ctx* c, const int32_t* row_ptr, const int32_t* col,
           }
         }
         if (wb == 4) {
-          NPS_CUDA(cudaMemcpyAsync(c->g_w.p, w, sizeof(uint32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
+          if ((e = copy_in(c, c->g_w.p, w, sizeof(uint32_t) * (size_t)m, s))) return e;
         } else {
           if ((e = c->g_wpack.ensure((size_t)wb * (size_t)m, false, s))) return e;
           NPS_CUDA(cudaMemcpyAsync(c->g_wpack.p, c->h_wpack, (size_t)wb * (size_t)m, cudaMemcpyHostToDevice, s));
@@ -847,8 +941,7 @@ nps_status sssp_ctx_impl(nps_ctx* c, const int32_t* row_ptr, const int32_t* col,
     bfs_levels_kernel<<<lg, 256, 0, s>>>(ddist, n);
     NPS_CUDA(cudaGetLastError());
   }
-  if (!p.device_ptrs)
-    NPS_CUDA(cudaMemcpyAsync(dist_out, ddist, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToHost, s));
+  if (!p.device_ptrs && (e = copy_out(c, dist_out, ddist, sizeof(uint32_t) * (size_t)n, s))) return e;
   NPS_CUDA(cudaEventRecord(c->ev[3], s));
   NPS_CUDA(cudaStreamSynchronize(s));
   const Counters& k = *c->h_ctr;
