@@ -89,6 +89,9 @@ constexpr int kHopRounds = 32;
 // Rounds then pause for kHopPause iterations, twice as many each time.  R-MAT 15, edge
 // factor 8, block level, unordered: 0.23 ms a call without rounds, 0.32 without the pause.
 constexpr uint32_t kHopPause = 8;
+// Breadth-first levels in step (InstDesc::bits) run CTA rounds, which make levels tentative,
+// only from this iteration on: a frontier still small then is a long graph's.
+constexpr uint32_t kBitsHopFrom = 4;
 constexpr int32_t kHopList = 128;
 
 // Per-instance device counters.  Zeroed by the host before a launch.
@@ -177,6 +180,8 @@ struct InstDesc {
   int32_t order_degree; // rows below this degree ignore the bucket bound (0 = none)
   uint32_t dsched;      // per-bucket log2 widths, 4 bits each (0 = fixed delta)
   int32_t sort_push;    // grid-tier rows sorted at push: 1 on, -1 off, 0 by the grid threshold
+  uint32_t* vis;        // breadth-first levels in step (bits): one bit per vertex with a level
+  int32_t bits;
   int32_t async;        // 1: buckets are processed without per-iteration barriers (GRID tiers)
   unsigned long long* nq;  // near ring: slot = (tag << 32) | vertex, tag = index + 1 when filled
   uint32_t nq_mask;        // ring capacity - 1 (a power of two)
@@ -413,6 +418,7 @@ struct IterCtx {
   bool early;            // near pushes of at least t_grid edges join this iteration's grid-tier
                          // list when their staging buffer is flushed (walked next iteration)
   bool want_hist;        // policy features or trace: count the degrees of those rows
+  bool bits;             // breadth-first levels in step: a vertex's first level is its last
 };
 
 // Whether an edge of weight w is relaxed by a pass over light (heavy = false)
@@ -513,6 +519,42 @@ __device__ __forceinline__ void relax_batch(const InstDesc& I, const IterCtx& C,
                                             bool (&pf)[K], Acc& acc) {
   uint32_t cur[K];
   bool go[K];
+  if (C.bits) {
+    // Levels in step: every vertex of the frontier has the same level, so the first edge
+    // to reach a vertex gives it its level.  The check reads one bit per vertex (0.5 MB at
+    // R-MAT 22, of which L1 holds much) instead of its distance (16 MB), and one atomicOr
+    // decides in place of an atomicMin and a stamp.
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      go[j] = valid[j];
+      if (valid[j]) {
+        acc.edges++;
+        if ((uint32_t)v[j] >= (uint32_t)I.n) {  // neighbour id outside [0, n): record and skip
+          atomicCAS(&I.ctr->status, 0u, (uint32_t)NPS_ERR_FORMAT);
+          go[j] = false;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) cur[j] = go[j] ? ld_dist(I.vis + ((uint32_t)v[j] >> 5)) : 0u;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint32_t bit = 1u << (v[j] & 31);
+      go[j] = go[j] && !(cur[j] & bit);
+      cur[j] = go[j] ? atomicOr(I.vis + ((uint32_t)v[j] >> 5), bit) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      pf[j] = false;
+      pn[j] = go[j] && !(cur[j] & (1u << (v[j] & 31)));
+      if (pn[j]) {
+        I.dist[v[j]] = nd[j];
+        acc.impr++;
+        acc.reached++;
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < K; ++j) {
     go[j] = valid[j];
@@ -912,6 +954,7 @@ struct Smem {
                                  // this round and the next
   };
   HopArgs hop_args;            // CTA rounds: the iteration, written by thread 0
+  int32_t bits_on;             // levels in step so far (InstDesc::bits)
   uint32_t hop_seeds;          // CTA rounds: frontier vertices per CTA up to which they run
   uint32_t hop_it, hop_from, hop_pause;  // CTA rounds: last iteration of rounds; the first one they
                                // may run in next; how long they pause when rows were listed
@@ -1754,7 +1797,7 @@ static __device__ __noinline__ bool agree_step(Counters* ctr, uint32_t it, uint3
 // frontier in q[0] (the source, or the state form's flagged vertices), a team
 // barrier, then the first bucket's width and level (from the policy's start state
 // when the learned policy runs).  Returns false when the run must stop.
-template <int BS>
+template <int BS, bool BITS>
 __device__ bool start_instance(const LaunchParams& P, const InstDesc& I, Smem<BS>& sm, uint32_t* bar,
                                uint32_t& bar_epoch, uint32_t rank, uint32_t team_size, bool& inject, bool learned,
                                uint32_t& base_out, uint32_t& qlen, uint32_t& delta, int& level) {
@@ -1769,6 +1812,7 @@ __device__ bool start_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     for (uint32_t v = gtid; v < (uint32_t)I.n; v += gthreads) {
       I.dist[v] = (v == (uint32_t)I.src) ? 0u : kInf;
       if (wrap) { I.mark[v] = 0; I.fmark[v] = 0; I.smark[v] = 0; }
+      if (BITS && (v & 31u) == 0) I.vis[v >> 5] = (v >> 5) == ((uint32_t)I.src >> 5) ? 1u << (I.src & 31) : 0u;
       if ((v & 7u) == 0) {
         // the stamps and row offsets are read at random for the whole run: bring them into
         // L2 with the evict-last priority while the distances are written (R-MAT 22: DRAM
@@ -1851,7 +1895,7 @@ __device__ bool start_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
 // ---------------------------------------------------------------------------
 // Solve one instance with the CTAs of one team.  I refers to kernel-parameter
 // space (single-instance launches) or to a shared-memory copy (batches).
-template <int BS, bool LEAN>
+template <int BS, bool LEAN, bool BITS>
 __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS>& sm, uint32_t* bar,
                                uint32_t& bar_epoch, uint32_t rank, uint32_t team_size, bool& inject) {
   constexpr int NW = BS / 32;
@@ -1868,10 +1912,11 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     sm.hop_it = 0xffffffffu;
     sm.hop_from = 0;
     sm.hop_pause = kHopPause;
+    sm.bits_on = BITS;
     sm.hop_seeds = max(1u, min(kHopSeeds, (uint32_t)((unsigned long long)kHopSeedEdges * (uint32_t)I.n /
                                                      (uint32_t)max(I.m, 1))));
   }
-  if (!start_instance<BS>(P, I, sm, bar, bar_epoch, rank, team_size, inject, learned, base, qlen, delta, level))
+  if (!start_instance<BS, BITS>(P, I, sm, bar, bar_epoch, rank, team_size, inject, learned, base, qlen, delta, level))
     return;
   uint32_t it = 0, ep = 0;
   uint32_t T = delta == 0 ? 0xffffffffu : delta;
@@ -1924,6 +1969,8 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
               (I.sort_push > 0 ||
                (I.sort_push == 0 && C.t_grid <= NPS_SORT_AT_PUSH_AUTO_MAX && I.w != nullptr));
     C.want_hist = want_iter;
+    C.bits = BITS && sm.bits_on;
+    if (BITS && C.bits) C.early = C.t_grid != 0x7fffffff;  // every row of a level in one iteration
     const int4* Hprev = I.heavy + ((it & 1) ? 0 : hhalf);
     const int32_t* Hitem = I.hitem + ((it & 1) ? 0 : I.icap);
 
@@ -1959,9 +2006,11 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     // the far pile and the settle list, nor where a pass per frontier is asked for: the
     // policy's and the trace's per-iteration statistics, degree ordering, local rounds.
     const bool hops = !advance && !heavy_it && !want_iter && hprev_tot == 0 && C.local_rounds == 0 &&
-                      C.order_deg == 0 && qlen <= team_size * sm.hop_seeds && it >= sm.hop_from;
+                      C.order_deg == 0 && qlen <= team_size * sm.hop_seeds && it >= sm.hop_from &&
+                      (!BITS || !C.bits || it >= kBitsHopFrom);
     if (hops && threadIdx.x == 0) {
       sm.hop_it = it;
+      sm.bits_on = 0;  // levels are tentative from here on
       const uint32_t per = max(kHopMinSeeds, (qlen + team_size - 1) / team_size);
       sm.hop_args.srcq = I.q[it & 1];
       sm.hop_args.begin = min(qlen, rank * per);
@@ -2316,7 +2365,7 @@ __device__ void solve_instance_async(const LaunchParams& P, const InstDesc& I, S
 
   uint32_t base = 0, srclen = 0, delta = 0;
   int level = 0;
-  if (!start_instance<BS>(P, I, sm, bar, bar_epoch, rank, team_size, inject, learned, base, srclen, delta, level))
+  if (!start_instance<BS, false>(P, I, sm, bar, bar_epoch, rank, team_size, inject, learned, base, srclen, delta, level))
     return;
   const int32_t* srcq = I.q[0];
   bool advance = false;
@@ -2353,6 +2402,7 @@ __device__ void solve_instance_async(const LaunchParams& P, const InstDesc& I, S
     C.sadd = nullptr;
     C.early = false;
     C.want_hist = false;
+    C.bits = false;
     if (rank == 0 && threadIdx.x == 0) {
       // slots of the next bucket (their last user ended two barriers ago)
       const uint32_t sl = (p + 1) % 3;
@@ -2685,10 +2735,10 @@ constexpr int kMinBlocks = BS >= 512 ? 2 : (BS >= 256 ? 3 : 6);
 // The persistent kernel.  SINGLE: one instance whose descriptor is the kernel
 // parameter `single` (constant-bank reads in the hot loops); otherwise the
 // team's instances are staged one at a time in shared memory.  LEAN: without the
-// optional orderings (nps_lean).  ASYNC (single
+// optional orderings (nps_lean).  BITS: breadth-first levels in step.  ASYNC (single
 // instances only): the asynchronous bucket schedule, in a kernel of its own so
 // that each schedule gets its own register allocation.
-template <int BS, bool SINGLE, bool ASYNC = false, bool LEAN = false>
+template <int BS, bool SINGLE, bool ASYNC = false, bool LEAN = false, bool BITS = false>
 __global__ void __launch_bounds__(BS, kMinBlocks<BS>) sssp_persistent_kernel(const __grid_constant__ LaunchParams P,
                                                              const __grid_constant__ InstDesc single) {
   __shared__ Smem<BS> sm;
@@ -2721,13 +2771,13 @@ __global__ void __launch_bounds__(BS, kMinBlocks<BS>) sssp_persistent_kernel(con
   if constexpr (SINGLE && ASYNC) {
     solve_instance_async<BS>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
   } else if constexpr (SINGLE) {
-    solve_instance<BS, LEAN>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
+    solve_instance<BS, LEAN, BITS>(P, single, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
   } else {
     for (int k = 0; k < td.inst_count; ++k) {
       __syncthreads();
       if (threadIdx.x == 0) sinst = P.inst[P.order[td.inst_begin + k]];
       __syncthreads();
-      solve_instance<BS, LEAN>(P, sinst, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
+      solve_instance<BS, LEAN, false>(P, sinst, sm, bar, bar_epoch, rank, (uint32_t)td.cta_count, inject);
       if (ld_relaxed_u32(P.abort_flag)) return;
       // instances of a team are separated by a barrier so every CTA sees the previous one done
       if (!team_barrier<BS>(P, sm, bar, bar_epoch, (uint32_t)td.cta_count, &sinst.ctr->status, false)) return;

@@ -153,17 +153,18 @@ nps_status device_info(int dev, DevInfo* out) {
 using KernelFn = void (*)(const LaunchParams, const InstDesc);
 
 template <int BS>
-KernelFn pick_kernel_bs(bool single, bool async, bool lean) {
+KernelFn pick_kernel_bs(bool single, bool async, bool lean, bool bits) {
+  if (bits) return nps::sssp_persistent_kernel<BS, true, false, true, true>;
   if (async) return nps::sssp_persistent_kernel<BS, true, true>;
   if (single) return lean ? nps::sssp_persistent_kernel<BS, true, false, true> : nps::sssp_persistent_kernel<BS, true>;
   return lean ? nps::sssp_persistent_kernel<BS, false, false, true> : nps::sssp_persistent_kernel<BS, false>;
 }
 
-KernelFn pick_kernel(int bs, bool single, bool async, bool lean) {
+KernelFn pick_kernel(int bs, bool single, bool async, bool lean, bool bits) {
   switch (bs) {
-    case 128: return pick_kernel_bs<128>(single, async, lean);
-    case 256: return pick_kernel_bs<256>(single, async, lean);
-    case 512: return pick_kernel_bs<512>(single, async, lean);
+    case 128: return pick_kernel_bs<128>(single, async, lean, bits);
+    case 256: return pick_kernel_bs<256>(single, async, lean, bits);
+    case 512: return pick_kernel_bs<512>(single, async, lean, bits);
     default: return nullptr;
   }
 }
@@ -195,10 +196,10 @@ cudaError_t set_carveout(int dev, KernelFn k, int bs, int nb) {
 // Grid of the persistent kernel: its resident CTAs per SM, asked for (and the carveout
 // set) once per device and kernel.
 nps_status grid_size(int dev, const DevInfo& di, int bs, bool single, int ctas_per_sm, int* grid,
-                     bool async, bool lean) {
+                     bool async, bool lean, bool bits = false) {
   static std::mutex mu;
   static std::map<std::pair<int, const void*>, int> resident;
-  KernelFn k = pick_kernel(bs, single, async, lean);
+  KernelFn k = pick_kernel(bs, single, async, lean, bits);
   if (!k) return nps_fail(NPS_ERR_INVALID_ARG, "block_size must be 128, 256 or 512");
   int nb = 0;
   {
@@ -284,7 +285,7 @@ struct nps_ctx {
   DevInfo di;
   // per-instance workspace (single-instance calls)
   DevBuf<int32_t> q0, q1, f0, f1, s0, s1;
-  DevBuf<uint32_t> mark, fmark, smark, stamp;
+  DevBuf<uint32_t> mark, fmark, smark, stamp, vis;
   DevBuf<int4> heavy;
   // work rings of the asynchronous schedule (tags and head/tail persist across runs)
   DevBuf<unsigned long long> nq;
@@ -348,7 +349,7 @@ void ctx_release(nps_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto* b : {&c->q0, &c->q1, &c->f0, &c->f1, &c->s0, &c->s1, &c->g_row, &c->g_col, &c->b_pool, &c->b_order})
     b->release();
-  for (auto* b : {&c->mark, &c->fmark, &c->smark, &c->stamp, &c->g_w, &c->g_dist, &c->b_stamp}) b->release();
+  for (auto* b : {&c->mark, &c->fmark, &c->smark, &c->stamp, &c->vis, &c->g_w, &c->g_dist, &c->b_stamp}) b->release();
   c->heavy.release();
   c->nq.release();
   c->segs.release();
@@ -524,7 +525,7 @@ unsigned long long run_budget_ns(const nps_params& p) {
 
 nps_status launch(nps_ctx* c, cudaStream_t s, int bs, bool single, bool lean, int grid, const LaunchParams& lp,
                   const InstDesc& inst) {
-  KernelFn k = pick_kernel(bs, single, single && inst.async != 0, lean);
+  KernelFn k = pick_kernel(bs, single, single && inst.async != 0, lean, single && inst.bits != 0);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)bs);
@@ -552,6 +553,8 @@ nps_status status_from_device(uint32_t st) {
   }
 }
 
+constexpr int64_t kBitsMinEdges = 4000000;
+
 // Core single-instance run on device-resident arrays.
 nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int32_t* col, const uint32_t* w,
                       int32_t n, int64_t m, int32_t src, uint32_t* dist, uint8_t* update, int mode,
@@ -570,8 +573,16 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   uint32_t icap = 0, ishift = 0;
   nps_heavy_items(m, hcap / 2, 0, &icap, &ishift);
   if ((e = c->heavy.ensure(nps_heavy_slots(hcap, icap), false, s))) return e;
+  // Breadth-first levels from one source, unordered: in step, unless rows are kept out of
+  // the grid-tier list at push (a level would then take two iterations) or a pass per
+  // frontier is recorded.  On graphs of kBitsMinEdges on: R-MAT 22 0.627 -> 0.574 ms, R-MAT
+  // 20 0.252 -> 0.243 (block level 0.56 -> 0.41); below, sorting every pushed row costs more
+  // than the bits save (R-MAT 14 0.071 -> 0.078).
+  const bool bits = !w && mode == 0 && m >= kBitsMinEdges && p.delta == 0 && p.delta_schedule == 0 && p.policy == NPS_POLICY_PLAIN &&
+                    nps_lean(p) && !use_async(p) && !p.trace && p.sort_at_push >= 0;
+  if (bits && (e = c->vis.ensure((nn + 31) / 32, false, s))) return e;
   int grid = 0;
-  if ((e = grid_size(c->device, c->di, p.block_size, true, p.ctas_per_sm, &grid, use_async(p), nps_lean(p)))) return e;
+  if ((e = grid_size(c->device, c->di, p.block_size, true, p.ctas_per_sm, &grid, use_async(p), nps_lean(p), bits))) return e;
   Control ctl(1, 1, grid);
   if ((e = c->control.ensure(ctl.bytes(), false, s))) return e;
   ctl.base = c->control.p;
@@ -631,6 +642,8 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   d.trace_cap = p.trace ? (uint32_t)c->trace.n : 0;
   d.vec_ok = (((uintptr_t)col | (uintptr_t)w) & 15) == 0;
   fill_thresholds(p, d);
+  d.vis = bits ? c->vis.p : nullptr;
+  d.bits = bits;
   d.policy = nps_policy_for(p, m);  // the learned policy only where it gains
   if (st) st->policy_used = (uint32_t)d.policy;
   if (async) {
