@@ -1492,8 +1492,8 @@ __device__ __forceinline__ void walk_item(const InstDesc& I, const IterCtx& C, c
 // Out of line, its sums in shared memory: the item loop's register allocation does not
 // pay for it.  What bounds it: the latency of a round, about 2,800 cycles for one vertex
 // (smem entry, edges beside the distance, atomicMin beside the head's row bounds, smem
-// push).  Measured (ms before -> after): 2,000-vertex path 13.6 -> 2.9; 2048 x 2048 grid,
-// delta 16384, 47.1 -> 14.3 and 4,984 -> 301 iterations; uniform 16,384 x 131,072, delta
+// push).  Measured (ms before -> after): 2,000-vertex path 13.6 -> 2.7; 2048 x 2048 grid,
+// delta 16384, 47.1 -> 14.1 and 4,984 -> 301 iterations; uniform 16,384 x 131,072, delta
 // 64, 0.318 -> 0.169; R-MAT 20 and 22 unchanged.
 // kHopEdges edges per lane (heads nb, weights in nd) of rows at distances du (kInf: the
 // row is skipped).  Every edge goes straight to its atomicMin: the distance check before
@@ -1634,14 +1634,20 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
     // the rows' edges, flat over the warp; long rows are listed below
     const bool lng = q.w - q.z >= t_list;
     const uint32_t d = lng ? 0u : (uint32_t)(q.w - q.z);
-    uint32_t incl = d;
+    // up to four entries of up to eight edges: eight lanes each, without a search (path
+    // 2.90 -> 2.72 ms, the grid at delta 4096 19.2 -> 18.6)
+    const bool eight = per <= 4 && __all_sync(kFull, d <= 8);
+    uint32_t total = 0, excl = 0;
+    if (!eight) {
+      uint32_t incl = d;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += t;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+      }
+      total = __shfl_sync(kFull, incl, 31);
+      excl = incl - d;
     }
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    const uint32_t excl = incl - d;
     uint32_t seen = sstamp;
     for (uint32_t k0 = 0; k0 == 0 || k0 < total; k0 += 32 * kHopEdges) {
       int32_t nb[kHopEdges];
@@ -1654,6 +1660,18 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
         nd[j] = 0u;
         go[j] = false;
         own[j] = 0;
+        if (eight && j == 0) {
+          const int o = lane >> 3;
+          const int32_t so = __shfl_sync(kFull, q.z, o);
+          const uint32_t dd = __shfl_sync(kFull, d, o), k = lane & 7;
+          own[j] = o;
+          go[j] = k < dd;
+          if (go[j]) {
+            nb[j] = __ldg(col + so + k);
+            nd[j] = wts ? __ldg(wts + so + k) : 1u;
+          }
+          continue;
+        }
         if (k0 + 32 * j >= total) continue;  // the whole warp
         const uint32_t k = k0 + 32 * j + lane;
         int o = 0;

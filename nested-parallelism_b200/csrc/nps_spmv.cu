@@ -422,8 +422,8 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_
 __global__ void __launch_bounds__(kThreads, kChunkCtas) spmv_chunks_kernel(Mat A, Lists L, double* part,
                                                                SpmvCtr* c) {
   cudaGridDependencySynchronize();  // launched ahead of the row pass's end, which it waits for here
-  if (c->status) return;            // the lists may have holes
-  const uint32_t nc = min((uint32_t)c->list, L.chunks);
+  const uint32_t bad = c->status, nc = min((uint32_t)c->list, L.chunks);  // read together
+  if (bad) return;  // the lists may have holes
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * kWarps;
   uint32_t q = blockIdx.x * kWarps + (threadIdx.x >> 5);
