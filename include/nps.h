@@ -412,9 +412,10 @@ typedef struct nps_instance {
 
 /* Run `count` independent instances in one persistent cooperative launch; CTAs
  * are split into teams (one team per group of instances, sized by edge count).
- * The first calls on an instance set form its teams and launch directly; with
- * use_graph = 1 the first call that repeats a set's launch unchanged captures it
- * into a CUDA graph, which later calls with the same set replay. */
+ * The first two calls on an instance set form its teams and launch directly; with
+ * use_graph = 1 the third, whose teams stay, captures the launch into a CUDA graph,
+ * which later calls with the same set replay (with more instances than CTAs, whose
+ * teams stay from the start, the second call captures). */
 nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, const nps_params* p,
                           int32_t use_graph, nps_stats* per_instance, float* kernel_ms);
 

@@ -1080,10 +1080,10 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
                         memcmp(&c->b_params_key, &p, sizeof(p)) == 0;
   const int nteams = std::min(count, grid);
   if (!same_set || nteams != count) c->b_stage = 0;
-  // stages 1 and 2 form the teams anew; stage 3 keeps the last split.  Calls that form
-  // teams launch directly: a graph pays for its capture and instantiation (about 0.2 ms
-  // for 64 instances) only when the launch is repeated as it is, so it is captured by the
-  // first call that repeats one.
+  // stages 1 and 2 form the teams anew; stage 3 keeps the last split.  A graph pays for its
+  // capture and instantiation (about 0.2 ms for 64 instances) only when the launch is
+  // repeated as it is: it is captured with the last split, or, where teams are not
+  // re-balanced, by the first call that repeats a launch.
   const bool rebalance = c->b_stage == 1 || c->b_stage == 2;
   const bool same = same_set && c->b_built && !rebalance;
   Control ctl((size_t)count, (size_t)nteams, grid);
@@ -1257,7 +1257,7 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
   if ((e = ensure_pinned_counters(c, (size_t)count))) return e;
 
   NPS_CUDA(cudaEventRecord(c->ev[1], s));
-  if (use_graph && same) {
+  if (use_graph && (same || c->b_stage >= 2)) {
     if (!c->b_graph) {
       cudaGraph_t g = nullptr;
       NPS_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
