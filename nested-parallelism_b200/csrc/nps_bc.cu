@@ -504,11 +504,14 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
               __syncwarp();
               flush(0, 32);
               if (have >= 64) flush(32, 32);
+              // those left move down: no store beyond them, where the next step's heads go, and
+              // a barrier before other lanes store those (a ballot alone orders no memory)
               const uint32_t done = have & ~31u;
-              const int32_t y = head[done + lane < 96u ? done + lane : 95u];
-              __syncwarp();
-              head[lane] = y;
               have -= done;
+              const int32_t y = (uint32_t)lane < have ? head[done + lane] : 0;
+              __syncwarp();
+              if ((uint32_t)lane < have) head[lane] = y;
+              __syncwarp();
             }
           }
           __syncwarp();
