@@ -2028,7 +2028,6 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
                       (!BITS || !C.bits || it >= kBitsHopFrom);
     if (hops && threadIdx.x == 0) {
       sm.hop_it = it;
-      sm.bits_on = 0;  // levels are tentative from here on
       const uint32_t per = max(kHopMinSeeds, (qlen + team_size - 1) / team_size);
       sm.hop_args.srcq = I.q[it & 1];
       sm.hop_args.begin = min(qlen, rank * per);
@@ -2051,6 +2050,9 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     const uint32_t srclen = advance ? adv_len : (heavy_it ? slen : qlen);
     Acc acc = {0, 0, 0, 0};
     if (hops) {
+      // levels are tentative from here on; every warp has read the flag for this iteration
+      // before the barrier above, and reads it next behind the team barrier
+      if (BITS && threadIdx.x == 0) sm.bits_on = 0;
       cta_rounds<BS>(I, sm);
     } else {
       const uint32_t n_heavy_items = (uint32_t)((hprev_tot + (1ull << I.item_shift) - 1) >> I.item_shift);
