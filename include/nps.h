@@ -337,7 +337,10 @@ nps_status nps_spmv(const int32_t* row_ptr, const int32_t* col, const double* va
  * bit-identical to bc_cpu for the same source order (a NaN from wrapped path
  * counts is a NaN on both, with a different payload).  One CTA per source; the
  * call holds about 16 n bytes per CTA of the grid plus up to 2 GB of per-source
- * dependency rows.  Pointers (sources included) are host or device per
+ * dependency rows.  The reference's mark of unvisited vertices is level 9999, so a
+ * vertex on that level is taken again by every edge that leads to it; a source with
+ * more such visits than there is room for (n + 4,096 vertices in its order) ends the
+ * call with NPS_ERR_CAPACITY.  Pointers (sources included) are host or device per
  * p->device_ptrs; uses p->device and p->stream. */
 nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t m, const int32_t* sources,
                   int32_t nsrc, const nps_params* p, float* bc_out, nps_stats* st);

@@ -28,7 +28,11 @@
 //             over sources exactly.
 //
 // MAX_LEVEL = 9999 marks unvisited vertices as in the reference
-// (common/global.h:17).  Path counts wrap as the reference's int sums do; where
+// (common/global.h:17).  A vertex on level 9999 therefore still counts as unvisited there:
+// every edge from level 9998 takes it into the order again, and so do edges from later
+// levels, which move it behind themselves.  bc_sources_kernel keeps that; the
+// shared-memory kernel, which marks vertices apart from their levels, stops at the first
+// vertex on level 9999, and the call runs bc_sources_kernel instead.  Path counts wrap as the reference's int sums do; where
 // that gives 0 / 0 the result is NaN on both sides, but with different payloads
 // (x86 writes 0xFFC00000, the GPU 0x7FFFFFFF), so NaNs match as NaNs only.
 #include <cuda_runtime.h>
@@ -49,6 +53,10 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int32_t kMaxLevel = 9999;
+// Order entries beyond n for vertices taken more than once (only in graphs of more than
+// kMaxLevel vertices); when they run out the call ends with NPS_ERR_CAPACITY.
+constexpr size_t kDeepSlack = 4096;
+__host__ __device__ constexpr size_t bc_order_entries(size_t n) { return n + (n > (size_t)kMaxLevel ? kDeepSlack : 0); }
 constexpr int32_t kWarpRow = 32;  // rows of at least this many edges are walked by a warp (forward)
 
 struct BcArgs {
@@ -61,10 +69,10 @@ struct BcArgs {
   int32_t count;
   int32_t* level;          // per CTA: n entries each
   int32_t* sigma;
-  int32_t* order;
-  int32_t* lb;             // per CTA: n + 2 level bounds
+  int32_t* order;          // per CTA: bc_order_entries(n) each
+  int32_t* lb;             // per CTA: bc_order_entries(n) + 2 level bounds
   float* delta;            // count rows of n
-  uint32_t* status;
+  uint32_t* status;        // an error, and [1]: the shared-memory kernel met level kMaxLevel
 };
 
 __device__ __forceinline__ void flag_format(uint32_t* status) { atomicCAS(status, 0u, (uint32_t)NPS_ERR_FORMAT); }
@@ -82,7 +90,7 @@ __device__ __forceinline__ bool row_ok(const BcArgs& a, int32_t u, int32_t& s, i
 
 // Forward relaxation of edge k from a vertex of level L with path count su.
 __device__ __forceinline__ void forward_edge(const BcArgs& a, int32_t* level, int32_t* sigma, int32_t* order,
-                                             int* s_tail, int64_t k, int32_t L, int32_t su) {
+                                             int32_t cap, int* s_tail, int64_t k, int32_t L, int32_t su) {
   const int32_t v = __ldg(a.col + k);
   if ((uint32_t)v >= (uint32_t)a.n) {
     flag_format(a.status);
@@ -93,7 +101,9 @@ __device__ __forceinline__ void forward_edge(const BcArgs& a, int32_t* level, in
     lv = atomicCAS(level + v, kMaxLevel, L + 1);
     if (lv == kMaxLevel) {
       lv = L + 1;
-      order[atomicAdd(s_tail, 1)] = v;
+      const int32_t i = atomicAdd(s_tail, 1);
+      if (i < cap) order[i] = v;
+      else atomicCAS(a.status, 0u, (uint32_t)NPS_ERR_CAPACITY);
     }
   }
   if (lv == L + 1) atomicAdd(sigma + v, su);  // wraps as the reference's int sum does
@@ -107,8 +117,9 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
   const size_t n = (size_t)a.n;
   int32_t* level = a.level + blockIdx.x * n;
   int32_t* sigma = a.sigma + blockIdx.x * n;
-  int32_t* order = a.order + blockIdx.x * n;
-  int32_t* lb = a.lb + blockIdx.x * (n + 2);
+  const int32_t cap = (int32_t)bc_order_entries(n);
+  int32_t* order = a.order + blockIdx.x * (size_t)cap;
+  int32_t* lb = a.lb + blockIdx.x * ((size_t)cap + 2);
   int sweep = 0;  // the same count in every thread
   if (tid == 0) s_nbig[0] = s_nbig[1] = 0;
   for (int j = blockIdx.x; j < a.count; j += gridDim.x) {
@@ -140,7 +151,7 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
               s_big[atomicAdd(&s_nbig[par], 1)] = u;  // at most one per thread per sweep
             } else {
               const int32_t su = __ldcg(sigma + u);
-              for (int64_t k = rs; k < re; ++k) forward_edge(a, level, sigma, order, &s_tail, k, L, su);
+              for (int64_t k = rs; k < re; ++k) forward_edge(a, level, sigma, order, cap, &s_tail, k, L, su);
             }
           }
         }
@@ -151,12 +162,12 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
           const int32_t u = s_big[b];
           const int32_t rs = a.row[u], re = a.row[u + 1];  // checked when listed
           const int32_t su = __ldcg(sigma + u);
-          for (int64_t k = (int64_t)rs + lane; k < re; k += 32) forward_edge(a, level, sigma, order, &s_tail, k, L, su);
+          for (int64_t k = (int64_t)rs + lane; k < re; k += 32) forward_edge(a, level, sigma, order, cap, &s_tail, k, L, su);
         }
         __syncthreads();
       }
       __syncthreads();
-      if (tid == 0) lb[L + 2] = s_tail;
+      if (tid == 0) lb[L + 2] = min(s_tail, cap);
       __syncthreads();
       ++L;
     }
@@ -184,7 +195,7 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
       __syncthreads();
     }
     // ---- leave the scratch as found: every reached vertex back to unvisited
-    const int32_t reached = s_tail;
+    const int32_t reached = min(s_tail, cap);
     for (int32_t i = tid; i < reached; i += kThreads) {
       const int32_t v = __ldcg(order + i);
       level[v] = kMaxLevel;
@@ -295,7 +306,7 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
   constexpr int NW = NT / 32;
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ double s_dyn[];
-  __shared__ int s_tail, s_item[2];
+  __shared__ int s_tail, s_stop, s_item[2];
   __shared__ int32_t s_lb[kSmemBounds];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
@@ -356,14 +367,20 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
       set_bound(1, 1);
       s_tail = 1;
       s_item[0] = s_item[1] = 0;
+      s_stop = n > kMaxLevel && __ldcg(a.status + 1) != 0u;
     }
     __syncthreads();
+    if (s_stop) return;  // another source met level kMaxLevel
     int sweep = 0;  // levels walked: the item counter of a level is reset in the next one
     // ---- forward: the frontier is order[bound(L), bound(L + 1))
     int32_t L = 0;
     for (;; ++L, ++sweep) {
       const int32_t lo = bound(L), hi = bound(L + 1);
       if (lo >= hi) break;
+      if (L == kMaxLevel) {  // the whole CTA: the bounds are the same in every thread
+        if (tid == 0) atomicExch(a.status + 1, 1u);
+        return;
+      }
       if (tid == 0) s_item[(sweep + 1) & 1] = 0;
       const int per = min(32, (hi - lo + NW - 1) / NW), items = (hi - lo + per - 1) / per;
       for (;;) {
@@ -643,7 +660,7 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   if (!W->stream) NPS_CUDA_RETURN(cudaStreamCreateWithFlags(&W->stream, cudaStreamNonBlocking));
   if (!W->ev[0])
     for (auto& ev : W->ev) NPS_CUDA_RETURN(cudaEventCreate(&ev));
-  if (!W->status) NPS_CUDA_RETURN(cudaMalloc((void**)&W->status, sizeof(uint32_t)));
+  if (!W->status) NPS_CUDA_RETURN(cudaMalloc((void**)&W->status, 2 * sizeof(uint32_t)));
   if (!W->sms) NPS_CUDA_RETURN(cudaDeviceGetAttribute(&W->sms, cudaDevAttrMultiProcessorCount, p.device));
   cudaStream_t s = p.stream ? (cudaStream_t)p.stream : W->stream;
   if (st) memset(st, 0, sizeof(*st));
@@ -668,35 +685,15 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
     dcol = W->col;
     dbc = W->bc;
   }
-  // one CTA per source at a time, as many CTAs as are resident; a block of
-  // sources shares one delta buffer
-  int threads = 0;  // of the shared-memory kernel; 0: the graph does not fit
-  const BcKernel smem_kernel = bc_pick_smem((size_t)n, p.device, &threads);
-  if (smem_kernel)
-    NPS_CUDA_RETURN(cudaFuncSetAttribute((const void*)smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)bc_smem_bytes((size_t)n, threads)));
-  const BcKernel kernel = smem_kernel ? smem_kernel : bc_sources_kernel;
-  const size_t dyn = smem_kernel ? bc_smem_bytes((size_t)n, threads) : 0;
-  if (!smem_kernel) threads = kThreads;
-  int per_sm = 0;
-  NPS_CUDA_RETURN(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, threads, dyn));
-  const size_t per_cta = smem_kernel ? (size_t)n + 2 : 4 * (size_t)n + 2;
-  // at most 8 GB of CTA scratch (16 n bytes each): large graphs run fewer sources at once
-  const int64_t by_memory = std::max<int64_t>(W->sms, (int64_t)((8ull << 30) / (per_cta * sizeof(int32_t))));
-  const int grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(std::min<int64_t>((int64_t)W->sms * std::max(1, per_sm), by_memory), count_all));
-  if ((e = nps_ensure(&W->scratch, &W->scratch_n, per_cta * (size_t)grid, s, "bc"))) return e;
-  const size_t budget = (size_t)1 << 31;  // bytes of delta rows per block
-  int64_t cap = std::max<int64_t>(grid, budget / (4 * (size_t)n));
-  if (p.reserved[1] > 0) cap = p.reserved[1];
-  const int32_t block = (int32_t)std::max<int64_t>(1, std::min<int64_t>(count_all, cap));
-  if ((e = nps_ensure(&W->delta, &W->delta_n, (size_t)block * (size_t)n, s, "bc"))) return e;
-  NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, sizeof(uint32_t), s));
-  NPS_CUDA_RETURN(cudaMemsetAsync(dbc, 0, sizeof(float) * (size_t)n, s));
-  if (dsrc && nsrc > 0 && p.device_ptrs) {
+  if (dsrc && nsrc > 0 && p.device_ptrs) {  // a bad device-side source list stops the call before any kernel reads it
+    uint32_t bad = 0;
+    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 2 * sizeof(uint32_t), s));
     bc_check_sources_kernel<<<(int)std::min<int64_t>(1024, ((int64_t)nsrc + 255) / 256), 256, 0, s>>>(dsrc, nsrc, n,
                                                                                                W->status);
     NPS_CUDA_RETURN(cudaGetLastError());
+    NPS_CUDA_RETURN(cudaMemcpyAsync(&bad, W->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    NPS_CUDA_RETURN(cudaStreamSynchronize(s));
+    if (bad) return nps_fail(NPS_ERR_INVALID_ARG, "bc: source out of range");
   }
   BcArgs a;
   a.row = drow;
@@ -704,50 +701,75 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   a.n = n;
   a.m = m;
   a.sources = dsrc;
-  if (smem_kernel) {
-    a.level = a.sigma = a.order = nullptr;
-    a.lb = W->scratch;
-  } else {
-    a.level = W->scratch;
-    a.sigma = W->scratch + (size_t)n * grid;
-    a.order = W->scratch + 2 * (size_t)n * grid;
-    a.lb = W->scratch + 3 * (size_t)n * grid;
-  }
-  a.delta = W->delta;
   a.status = W->status;
-  if (!smem_kernel) {
-    bc_fill_kernel<<<W->sms * 4, 256, 0, s>>>(a.level, a.sigma, (size_t)n * grid);
-    NPS_CUDA_RETURN(cudaGetLastError());
-  }
-  uint32_t h_status = 0;
-  if (dsrc && p.device_ptrs) {  // a bad device-side source list stops the call before any kernel reads it
-    NPS_CUDA_RETURN(cudaMemcpyAsync(&h_status, W->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  // one CTA per source at a time, as many CTAs as are resident; a block of
+  // sources shares one delta buffer
+  int smem_threads = 0;
+  BcKernel smem_kernel = bc_pick_smem((size_t)n, p.device, &smem_threads);
+  uint32_t h_status[2];
+  int grid = 0;
+  for (bool first = true;; first = false) {
+    const BcKernel kernel = smem_kernel ? smem_kernel : bc_sources_kernel;
+    const int threads = smem_kernel ? smem_threads : kThreads;
+    const size_t dyn = smem_kernel ? bc_smem_bytes((size_t)n, threads) : 0;
+    if (smem_kernel)
+      NPS_CUDA_RETURN(cudaFuncSetAttribute((const void*)smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    int per_sm = 0;
+    NPS_CUDA_RETURN(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, threads, dyn));
+    const size_t ordered = bc_order_entries((size_t)n);
+    const size_t per_cta = smem_kernel ? (size_t)n + 2 : 2 * (size_t)n + 2 * ordered + 2;
+    // at most 8 GB of CTA scratch (16 n bytes each): large graphs run fewer sources at once
+    const int64_t by_memory = std::max<int64_t>(W->sms, (int64_t)((8ull << 30) / (per_cta * sizeof(int32_t))));
+    grid = (int)std::max<int64_t>(
+        1, std::min<int64_t>(std::min<int64_t>((int64_t)W->sms * std::max(1, per_sm), by_memory), count_all));
+    if ((e = nps_ensure(&W->scratch, &W->scratch_n, per_cta * (size_t)grid, s, "bc"))) return e;
+    const size_t budget = (size_t)1 << 31;  // bytes of delta rows per block
+    int64_t cap = std::max<int64_t>(grid, budget / (4 * (size_t)n));
+    if (p.reserved[1] > 0) cap = p.reserved[1];
+    const int32_t block = (int32_t)std::max<int64_t>(1, std::min<int64_t>(count_all, cap));
+    if ((e = nps_ensure(&W->delta, &W->delta_n, (size_t)block * (size_t)n, s, "bc"))) return e;
+    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 2 * sizeof(uint32_t), s));
+    NPS_CUDA_RETURN(cudaMemsetAsync(dbc, 0, sizeof(float) * (size_t)n, s));
+    if (smem_kernel) {
+      a.level = a.sigma = a.order = nullptr;
+      a.lb = W->scratch;
+    } else {
+      a.level = W->scratch;
+      a.sigma = a.level + (size_t)n * grid;
+      a.order = a.sigma + (size_t)n * grid;
+      a.lb = a.order + ordered * grid;
+      bc_fill_kernel<<<W->sms * 4, 256, 0, s>>>(a.level, a.sigma, (size_t)n * grid);
+      NPS_CUDA_RETURN(cudaGetLastError());
+    }
+    a.delta = W->delta;
+    if (first) NPS_CUDA_RETURN(cudaEventRecord(W->ev[1], s));
+    const int fold_grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)W->sms * 8));
+    for (int32_t base = 0; base < count_all; base += block) {
+      a.src_base = base;
+      a.count = std::min<int32_t>(block, count_all - base);
+      kernel<<<grid, threads, dyn, s>>>(a);
+      NPS_CUDA_RETURN(cudaGetLastError());
+      bc_fold_kernel<<<fold_grid, 256, 0, s>>>(dbc, W->delta, n, a.count);
+      NPS_CUDA_RETURN(cudaGetLastError());
+    }
+    NPS_CUDA_RETURN(cudaEventRecord(W->ev[2], s));
+    if (!p.device_ptrs) NPS_CUDA_RETURN(cudaMemcpyAsync(bc_out, dbc, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s));
+    NPS_CUDA_RETURN(cudaMemcpyAsync(h_status, W->status, sizeof(h_status), cudaMemcpyDeviceToHost, s));
+    NPS_CUDA_RETURN(cudaEventRecord(W->ev[3], s));
     NPS_CUDA_RETURN(cudaStreamSynchronize(s));
-    if (h_status) return nps_fail(NPS_ERR_INVALID_ARG, "bc: source out of range");
+    if (!smem_kernel || !h_status[1]) break;
+    smem_kernel = nullptr;  // levels up to kMaxLevel: again, with the kernel that counts as the reference does
   }
-  NPS_CUDA_RETURN(cudaEventRecord(W->ev[1], s));
-  const int fold_grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)W->sms * 8));
-  for (int32_t base = 0; base < count_all; base += block) {
-    a.src_base = base;
-    a.count = std::min<int32_t>(block, count_all - base);
-    kernel<<<grid, threads, dyn, s>>>(a);
-    NPS_CUDA_RETURN(cudaGetLastError());
-    bc_fold_kernel<<<fold_grid, 256, 0, s>>>(dbc, W->delta, n, a.count);
-    NPS_CUDA_RETURN(cudaGetLastError());
-  }
-  NPS_CUDA_RETURN(cudaEventRecord(W->ev[2], s));
-  if (!p.device_ptrs) NPS_CUDA_RETURN(cudaMemcpyAsync(bc_out, dbc, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s));
-  NPS_CUDA_RETURN(cudaMemcpyAsync(&h_status, W->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  NPS_CUDA_RETURN(cudaEventRecord(W->ev[3], s));
-  NPS_CUDA_RETURN(cudaStreamSynchronize(s));
   if (st) {
-    st->status = (int32_t)h_status;
+    st->status = (int32_t)h_status[0];
     st->grid_ctas = grid;
     st->vertices_processed = (uint64_t)count_all;
     cudaEventElapsedTime(&st->kernel_ms, W->ev[1], W->ev[2]);
     cudaEventElapsedTime(&st->total_ms, W->ev[0], W->ev[3]);
   }
-  if (h_status == NPS_ERR_FORMAT)
+  if (h_status[0] == NPS_ERR_FORMAT)
     return nps_fail(NPS_ERR_FORMAT, "malformed CSR: a row range or column index is out of bounds");
+  if (h_status[0] == NPS_ERR_CAPACITY)
+    return nps_fail(NPS_ERR_CAPACITY, "bc: no room for the repeated visits of vertices on level 9999");
   return NPS_OK;
 }

@@ -307,8 +307,10 @@ int oracle_bc(int32_t n, const int32_t* row, const int32_t* col, int32_t nsrc, c
   int32_t* level = (int32_t*)malloc(sizeof(int32_t) * (size_t)n);
   int32_t* sigma = (int32_t*)malloc(sizeof(int32_t) * (size_t)n);
   float* delta = (float*)malloc(sizeof(float) * (size_t)n);
-  int32_t* order = (int32_t*)malloc(sizeof(int32_t) * (size_t)n);
-  int32_t* lb = (int32_t*)malloc(sizeof(int32_t) * ((size_t)n + 2));
+  /* a vertex on level 9999 still counts as unvisited and is appended again, at most once per edge */
+  const size_t most = (size_t)n + (n > ORACLE_MAX_LEVEL ? (size_t)row[n] : 0);
+  int32_t* order = (int32_t*)malloc(sizeof(int32_t) * most);
+  int32_t* lb = (int32_t*)malloc(sizeof(int32_t) * (most + 2));
   if (!level || !sigma || !delta || !order || !lb) {
     free(level), free(sigma), free(delta), free(order), free(lb);
     return -1;
