@@ -164,7 +164,9 @@ enum {
 };
 
 typedef struct nps_stats {
-  uint32_t iterations;      /* frontier iterations (the reference's `iteration` global) */
+  uint32_t iterations;      /* frontier iterations (the reference's `iteration` global): frontiers processed
+                               one after the other, counted along the CTA that followed most where CTAs
+                               follow small frontiers by themselves between two team barriers */
   uint32_t buckets;         /* near-far bucket advances */
   uint64_t edges_scanned;   /* edge relaxations attempted */
   uint64_t improvements;    /* successful atomicMin relaxations */
@@ -310,7 +312,7 @@ nps_status nps_sssp_noalloc(const int32_t* d_row_ptr, const int32_t* d_col, cons
  * count from src, NPS_BFS_UNDEFINED for unreachable vertices (bfs_rec.h:13); the
  * result equals the reference's bfs_cpu (apps/bfs-rec/src/gpu/bfs_rec.cpp:100-119).
  * Arguments as nps_sssp.  With unit weights the unordered frontier (delta 0)
- * already advances one level per iteration; delta = 1 gives one bucket per level. */
+ * already advances one level at a time; delta = 1 gives one bucket per level. */
 #define NPS_BFS_UNDEFINED 0x7FFFFFFF
 nps_status nps_bfs(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t m, int32_t src,
                    const nps_params* p, int32_t* level_out, nps_stats* st);

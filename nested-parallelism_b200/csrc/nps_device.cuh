@@ -102,7 +102,7 @@ struct __align__(128) Counters {
   uint32_t stail[3];   // settle-list tails, slot = heavy generation % 3
   uint32_t status;     // NPS_OK or the first error
   unsigned long long heavy[3];  // grid-tier list counter, slot = iteration % 3
-  uint32_t iterations;
+  uint32_t iterations; // of the team (a call's statistics count `rounds` too)
   uint32_t buckets;
   uint32_t reached;    // vertices whose distance left INF during the run
   uint32_t pad0;
@@ -127,7 +127,10 @@ struct __align__(128) Counters {
   // iteration may already be appending while a slower CTA decides: a bucket advance
   // appends the far-pile vertices it processes)
   uint32_t sadd[3];
-  uint32_t pad2[2];
+  // frontiers beyond the first that a CTA followed in its rounds of an iteration, the most
+  // of any CTA, slot = iteration % 3; and their sum over the iterations
+  uint32_t hop_more[3];
+  uint32_t rounds;
   // striped work counters, one 128-byte line each: work[slot][stripe * 32]
   // decision agreement: every CTA adds a hash of the counters its decision after iteration
   // i read to slot i % 4, and checks the sum one iteration later (team size x its own hash)
@@ -959,6 +962,7 @@ struct Smem {
   uint32_t hop_it, hop_from, hop_pause;  // CTA rounds: last iteration of rounds; the first one they
                                // may run in next; how long they pause when rows were listed
   uint32_t hop_n[3];           // CTA rounds: entries pushed for round r in hop_n[r % 3]
+  uint32_t hop_rounds;         // rank 0: sum of Counters::hop_more over the iterations
   unsigned long long hop_acc[4];         // CTA rounds: edges, improvements, first reaches, vertices of the solve
   int32_t stage[BS / 32][3][kStage];  // per-warp append staging: [near, far, settle]
   uint32_t red[4][BS / 32];
@@ -1723,6 +1727,7 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
   if (S.ncnt) stage_flush(S.nbuf, S.ncnt, S.ncnt, C.qn, C.qn_tail, I.qcap, status, lane);
   if (S.fcnt) stage_flush(S.fbuf, S.fcnt, S.fcnt, C.fp, C.fp_tail, I.qcap, status, lane);
   if (S.scnt) stage_flush(S.sbuf, S.scnt, S.scnt, C.sq, C.sq_tail, I.qcap, status, lane, C.sadd);
+  if (tid == 0 && r > 1) atomicMax(&I.ctr->hop_more[sm.hop_it % 3], (uint32_t)r - 1);
   const uint32_t a[4] = {__reduce_add_sync(kFull, acc.edges), __reduce_add_sync(kFull, acc.impr),
                          __reduce_add_sync(kFull, acc.reached), __reduce_add_sync(kFull, acc.processed)};
   if (lane == 0) {
@@ -1930,6 +1935,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
     sm.hop_it = 0xffffffffu;
     sm.hop_from = 0;
     sm.hop_pause = kHopPause;
+    sm.hop_rounds = 0;
     sm.bits_on = BITS;
     sm.hop_seeds = max(1u, min(kHopSeeds, (uint32_t)((unsigned long long)kHopSeedEdges * (uint32_t)I.n /
                                                      (uint32_t)max(I.m, 1))));
@@ -2000,6 +2006,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
         ctr->ftail[(E + 1) % 3] = 0;
         ctr->fmin[(E + 1) % 3] = 0xffffffffu;
         ctr->sadd[(it + 1) % 3] = 0;
+        ctr->hop_more[(it + 1) % 3] = 0;
         ctr->agree[(it + 1) % 4] = 0;  // last read by the decision after iteration it - 2
         if (heavy_it) ctr->stail[(hg + 1) % 3] = 0;
         if (want_iter) {
@@ -2205,6 +2212,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       const uint32_t f1 = __ldcg(&ctr->ftail[ep % 3]);
       const uint32_t m1 = __ldcg(&ctr->fmin[ep % 3]);
       const uint32_t s1 = __ldcg(&ctr->sadd[it % 3]);
+      const uint32_t hr = rank == 0 ? __ldcg(&ctr->hop_more[it % 3]) : 0u;
       const uint32_t st1 = ld_relaxed_u32(&ctr->status);
       uint32_t hb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       unsigned long long ie = 0, ii = 0;
@@ -2222,6 +2230,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       sm.bc_m = m1;
       sm.bc_s = s1;
       sm.bc_ag = ag;
+      sm.hop_rounds += hr;
       if (sm.hop_it == it && h1 != 0) {  // CTA rounds listed rows (every CTA read the same count)
         sm.hop_from = it + 1 + sm.hop_pause;
         sm.hop_pause *= 2;
@@ -2338,6 +2347,7 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
   if (threadIdx.x == 0) {
     if (rank == 0) {
       ctr->iterations = it;
+      ctr->rounds = sm.hop_rounds;
       ctr->solve_ns = globaltimer_ns() - sm.t_start;
       ctr->buckets = buckets;
       *I.stamp_base = base + (it > ep ? it : ep) + 4;
