@@ -355,7 +355,8 @@ nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t
  * none); st->iterations = the largest color (the reference's iteration count).
  * p->threshold is checked (at least 1); the kernel cuts long rows at lengths of its
  * own.  Pointers are host or device per p->device_ptrs; uses p->device, p->stream,
- * p->timeout_s (the bound on each wait for a color) and p->ctas_per_sm. */
+ * p->timeout_s (a wait for a color ends the call when for that long nothing moves)
+ * and p->ctas_per_sm. */
 nps_status nps_color(const int32_t* row_ptr, const int32_t* col, int32_t n, int64_t m, const nps_params* p,
                      int32_t* color_out, nps_stats* st);
 

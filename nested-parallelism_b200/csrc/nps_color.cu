@@ -21,7 +21,9 @@
 // of a long row does it).  A vertex waits only for smaller ids, whose units have smaller
 // tickets, each claimed by a warp that is running: the first unit not finished never
 // waits, so every wait ends, whatever is resident.  A color is one word, written once, so
-// no ordering between words is needed.  Each wait is bounded by timeout_s.
+// no ordering between words is needed.  Each wait is bounded: it ends the call when for
+// timeout_s neither its list shrinks nor any warp claims a unit, which each does when it
+// finishes one.
 //
 // What bounds it: the chain of dependent colors, each link a store and the poll that sees
 // it (R-MAT scale 22: 1,295 links, 1.6 us each), beside 33 M random 4-byte lookups, of
@@ -268,10 +270,12 @@ __global__ void __launch_bounds__(kThreads) color_units_kernel(ColorArgs a) {
   }
 }
 
-// A warp's wait: counted from the last time an entry left its list.
+// A warp's wait: counted from the last time an entry left its list or the ticket moved.
+// (The last of a window of vertices waits for the colors of all others: 18 ms on a path,
+// however short the timeout.)
 struct Wait {
   unsigned long long since;
-  uint32_t spins;
+  uint32_t spins, next;
 };
 
 // After a poll that changed nothing: true when the warp must stop, because this wait or
@@ -281,7 +285,9 @@ __device__ __forceinline__ bool wait_more(const ColorArgs& a, Wait& w, int lane)
     uint32_t quit = 0;
     if (lane == 0) {
       const unsigned long long now = globaltimer_ns();
-      if (w.since == 0) w.since = now;
+      const uint32_t next = ld_relaxed_u32(&a.c->next);
+      if (w.since == 0 || next != w.next) w.since = now;
+      w.next = next;
       quit = ld_relaxed_u32(&a.c->abort) != 0;
       if (!quit && now - w.since > a.timeout_ns) {
         atomicCAS(&a.c->status, 0u, (uint32_t)NPS_ERR_TIMEOUT);
@@ -324,7 +330,7 @@ __device__ __forceinline__ bool color_run(const ColorArgs& a, const Warp& W, int
   }
   const uint32_t excl = incl - d, total = __shfl_sync(kFull, incl, 31);
   __syncwarp();
-  Wait w = {0ull, 0u};
+  Wait w = {0ull, 0u, 0u};
   for (uint32_t k0 = 0;;) {
     if (!walked && incl <= k0) {  // this lane's row is walked
       atomicSub(&W.wait[lane], 1);
@@ -488,7 +494,7 @@ __device__ __forceinline__ bool color_chunk(const ColorArgs& a, const Warp& W, i
   __syncwarp();
   // all of them must have colors, in whatever order they get them: wait for kPoll entries
   // per lane at a time, so that a poll never goes over the whole list
-  Wait w = {0ull, 0u};
+  Wait w = {0ull, 0u, 0u};
   while (inject)
     if (wait_more(a, w, lane)) return false;
   for (uint32_t i0 = 0; i0 < len; i0 += 32 * kPoll) {
