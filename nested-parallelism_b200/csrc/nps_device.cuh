@@ -102,7 +102,7 @@ struct __align__(128) Counters {
   uint32_t stail[3];   // settle-list tails, slot = heavy generation % 3
   uint32_t status;     // NPS_OK or the first error
   unsigned long long heavy[3];  // grid-tier list counter, slot = iteration % 3
-  uint32_t iterations; // of the team (a call's statistics count `rounds` too)
+  uint32_t iterations; // of the team (iterations_of adds the rounds)
   uint32_t buckets;
   uint32_t reached;    // vertices whose distance left INF during the run
   uint32_t pad0;
@@ -137,6 +137,11 @@ struct __align__(128) Counters {
   uint32_t agree[4];
   alignas(128) uint32_t work[3][kStripes * 32];
 };
+
+// Frontiers processed one after the other: the team's iterations and the rounds in them.
+inline uint32_t iterations_of(const Counters& k) {
+  return k.iterations + k.rounds;
+}
 
 // Work rings of the asynchronous buckets.  Head and tail counters persist across
 // runs on a workspace (like the stamp base), each on its own 128-byte line.
@@ -962,6 +967,7 @@ struct Smem {
   uint32_t hop_it, hop_from, hop_pause;  // CTA rounds: last iteration of rounds; the first one they
                                // may run in next; how long they pause when rows were listed
   uint32_t hop_n[3];           // CTA rounds: entries pushed for round r in hop_n[r % 3]
+  uint32_t hop_last;           // CTA rounds: how many there were in the last iteration of rounds
   uint32_t hop_rounds;         // rank 0: sum of Counters::hop_more over the iterations
   unsigned long long hop_acc[4];         // CTA rounds: edges, improvements, first reaches, vertices of the solve
   int32_t stage[BS / 32][3][kStage];  // per-warp append staging: [near, far, settle]
@@ -1717,6 +1723,7 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
       stage_k<1>(S.sbuf, S.scnt, f, vv, sq, C.sq_tail, I.qcap, status, lane, nullptr, nullptr, C.sadd);
     }
   }
+  if (tid == 0) sm.hop_last = (uint32_t)r;
   // entries left: to the near queue
   for (uint32_t i0 = 0; i0 < cnt; i0 += BS) {
     const uint32_t i = i0 + tid;
@@ -1727,7 +1734,6 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
   if (S.ncnt) stage_flush(S.nbuf, S.ncnt, S.ncnt, C.qn, C.qn_tail, I.qcap, status, lane);
   if (S.fcnt) stage_flush(S.fbuf, S.fcnt, S.fcnt, C.fp, C.fp_tail, I.qcap, status, lane);
   if (S.scnt) stage_flush(S.sbuf, S.scnt, S.scnt, C.sq, C.sq_tail, I.qcap, status, lane, C.sadd);
-  if (tid == 0 && r > 1) atomicMax(&I.ctr->hop_more[sm.hop_it % 3], (uint32_t)r - 1);
   const uint32_t a[4] = {__reduce_add_sync(kFull, acc.edges), __reduce_add_sync(kFull, acc.impr),
                          __reduce_add_sync(kFull, acc.reached), __reduce_add_sync(kFull, acc.processed)};
   if (lane == 0) {
@@ -2061,6 +2067,8 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       // before the barrier above, and reads it next behind the team barrier
       if (BITS && threadIdx.x == 0) sm.bits_on = 0;
       cta_rounds<BS>(I, sm);
+      // (ordered before this CTA's arrival at the team barrier by its release)
+      if (threadIdx.x == 0 && sm.hop_last > 1) atomicMax(&ctr->hop_more[it % 3], sm.hop_last - 1);
     } else {
       const uint32_t n_heavy_items = (uint32_t)((hprev_tot + (1ull << I.item_shift) - 1) >> I.item_shift);
       // vertex items hold 32 frontier entries, or 16 / 8 / 4 when the frontier is small

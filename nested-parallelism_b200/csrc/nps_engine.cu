@@ -694,7 +694,7 @@ void reset_stamps(nps_ctx* c, cudaStream_t s) {
 
 void fill_stats(const Counters& k, nps_stats* st) {
   if (!st) return;
-  st->iterations = k.iterations + k.rounds;  // frontiers, one after the other
+  st->iterations = nps::iterations_of(k);
   st->buckets = k.buckets;
   st->edges_scanned = k.edges;
   st->improvements = k.improvements;

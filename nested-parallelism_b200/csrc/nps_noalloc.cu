@@ -257,7 +257,7 @@ extern "C" nps_status nps_sssp_noalloc(const int32_t* d_row_ptr, const int32_t* 
     NA_CUDA(cudaStreamSynchronize(s));
   }
   if (st) {
-    st->iterations = h.iterations + h.rounds;  // frontiers, one after the other
+    st->iterations = nps::iterations_of(h);
     st->buckets = h.buckets;
     st->edges_scanned = h.edges;
     st->improvements = h.improvements;
