@@ -1614,9 +1614,8 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
     sm.hop_n[0] = A.end - A.begin;
     sm.hop_n[1] = 0;
   }
-  // rows for the grid-tier list; its capacity counts rows of at least the smallest grid
-  // threshold of the parameters
-  const int32_t t_list = max(kHopList, I.level == NPS_LEVEL_HYBRID ? I.t3 : I.t1);
+  // rows for the grid-tier list, whose capacity counts rows from here on at every level
+  const int32_t t_list = max(kHopList, I.t1);
   uint32_t cnt;
   int r = 0;
   for (;; ++r) {
