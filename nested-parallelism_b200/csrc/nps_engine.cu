@@ -556,7 +556,23 @@ nps_status status_from_device(uint32_t st) {
   }
 }
 
-constexpr int64_t kBitsMinEdges = 4000000;
+// Edges from which a breadth-first run keeps its levels in step (none at the warp level: there
+// the first levels, which run no CTA rounds then, leave a hub's row to one warp.  R-MAT 20 at
+// edge factor 16, warp level: 1.87 ms in step, 1.12 not).  At the grid level every pushed row
+// is sorted, which only large graphs win back.  ms in step / not, defaults: uniform 1 M x 8 M
+// 0.214 / 0.190, 4 M x 16 M 0.502 / 0.483, 4 M x 40 M 0.537 / 0.558, 8 M x 64 M 0.966 / 0.998;
+// R-MAT 18 x 20 0.155 / 0.148, 20 x 8 0.201 / 0.207, 20 x 16 0.249 / 0.248, 21 x 16 0.355 /
+// 0.382, 22 x 16 0.577 / 0.635.  Block level, 256 threads, threshold 64: R-MAT 18 x 20 0.191 /
+// 0.205, 20 x 16 0.384 / 0.466, uniform 0.1 M x 4.1 M 0.088 / 0.093, 1 M x 8 M 0.179 / 0.181.
+// Hybrid level: R-MAT 18 x 20 0.175 / 0.183, 19 x 16 0.213 / 0.257, uniform 1 M x 8 M 0.184 /
+// 0.181.  Below 4 M edges: R-MAT 14 0.078 / 0.071.
+int64_t bits_min_edges(int level) {
+  switch (level) {
+    case NPS_LEVEL_WARP: return INT64_MAX;
+    case NPS_LEVEL_GRID: return 16000000;
+    default: return 4000000;
+  }
+}
 
 // Core single-instance run on device-resident arrays.
 nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int32_t* col, const uint32_t* w,
@@ -578,10 +594,8 @@ nps_status run_single(nps_ctx* c, cudaStream_t s, const int32_t* row, const int3
   if ((e = c->heavy.ensure(nps_heavy_slots(hcap, icap), false, s))) return e;
   // Breadth-first levels from one source, unordered: in step, unless rows are kept out of
   // the grid-tier list at push (a level would then take two iterations) or a pass per
-  // frontier is recorded.  On graphs of kBitsMinEdges on: R-MAT 22 0.627 -> 0.574 ms, R-MAT
-  // 20 0.252 -> 0.243 (block level 0.56 -> 0.41); below, sorting every pushed row costs more
-  // than the bits save (R-MAT 14 0.071 -> 0.078).
-  const bool bits = !w && mode == 0 && m >= kBitsMinEdges && p.delta == 0 && p.delta_schedule == 0 && p.policy == NPS_POLICY_PLAIN &&
+  // frontier is recorded; from bits_min_edges edges on.
+  const bool bits = !w && mode == 0 && m >= bits_min_edges(p.level) && p.delta == 0 && p.delta_schedule == 0 && p.policy == NPS_POLICY_PLAIN &&
                     nps_lean(p) && !use_async(p) && !p.trace && p.sort_at_push >= 0;
   if (bits && (e = c->vis.ensure((nn + 31) / 32, false, s))) return e;
   int grid = 0;
