@@ -30,14 +30,15 @@
 // MAX_LEVEL = 9999 marks unvisited vertices as in the reference
 // (common/global.h:17).  A vertex on level 9999 therefore still counts as unvisited there:
 // every edge from level 9998 takes it into the order again, and so do edges from later
-// levels, which move it behind themselves.  bc_sources_kernel keeps that; the
-// shared-memory kernel, which marks vertices apart from their levels, stops at the first
-// vertex on level 9999, and the call runs bc_sources_kernel instead.  Path counts wrap as the reference's int sums do; where
+// levels, which move it behind themselves.  bc_sources_kernel<true> keeps that, with room
+// for the repeated visits; the other kernels stop when a source gets that far, and the
+// call starts again with it.  Path counts wrap as the reference's int sums do; where
 // that gives 0 / 0 the result is NaN on both sides, but with different payloads
 // (x86 writes 0xFFC00000, the GPU 0x7FFFFFFF), so NaNs match as NaNs only.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -72,7 +73,9 @@ struct BcArgs {
   int32_t* order;          // per CTA: bc_order_entries(n) each
   int32_t* lb;             // per CTA: bc_order_entries(n) + 2 level bounds
   float* delta;            // count rows of n
-  uint32_t* status;        // an error, and [1]: the shared-memory kernel met level kMaxLevel
+  uint32_t* status;        // an error; [1]: the call starts again with another kernel (2: for level
+                           // kMaxLevel), [2]: sources found narrow
+  int32_t narrow;          // a source with fewer vertices than this up to level kLookLevel is narrow (0: none)
 };
 
 __device__ __forceinline__ void flag_format(uint32_t* status) { atomicCAS(status, 0u, (uint32_t)NPS_ERR_FORMAT); }
@@ -88,7 +91,9 @@ __device__ __forceinline__ bool row_ok(const BcArgs& a, int32_t u, int32_t& s, i
   return true;
 }
 
-// Forward relaxation of edge k from a vertex of level L with path count su.
+// Forward relaxation of edge k from a vertex of level L with path count su.  Below level
+// kMaxLevel a vertex enters the order once, so it has room; else (DEEP) `cap` entries.
+template <bool DEEP>
 __device__ __forceinline__ void forward_edge(const BcArgs& a, int32_t* level, int32_t* sigma, int32_t* order,
                                              int32_t cap, int* s_tail, int64_t k, int32_t L, int32_t su) {
   const int32_t v = __ldg(a.col + k);
@@ -102,13 +107,14 @@ __device__ __forceinline__ void forward_edge(const BcArgs& a, int32_t* level, in
     if (lv == kMaxLevel) {
       lv = L + 1;
       const int32_t i = atomicAdd(s_tail, 1);
-      if (i < cap) order[i] = v;
+      if (!DEEP || i < cap) order[i] = v;
       else atomicCAS(a.status, 0u, (uint32_t)NPS_ERR_CAPACITY);
     }
   }
   if (lv == L + 1) atomicAdd(sigma + v, su);  // wraps as the reference's int sum does
 }
 
+template <bool DEEP>
 __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
   __shared__ int s_tail;
   __shared__ int s_nbig[2];  // per sweep parity: a count is reset one sweep after its last read
@@ -131,7 +137,7 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
       sigma[s] = 1;
       order[0] = s;
       lb[0] = 0;
-      lb[1] = 1;
+      lb[1] = DEEP || a.n < kMaxLevel || __ldcg(a.status + 1) == 0u;  // no frontier when the call starts again
       s_tail = 1;
     }
     __syncthreads();
@@ -151,7 +157,7 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
               s_big[atomicAdd(&s_nbig[par], 1)] = u;  // at most one per thread per sweep
             } else {
               const int32_t su = __ldcg(sigma + u);
-              for (int64_t k = rs; k < re; ++k) forward_edge(a, level, sigma, order, cap, &s_tail, k, L, su);
+              for (int64_t k = rs; k < re; ++k) forward_edge<DEEP>(a, level, sigma, order, cap, &s_tail, k, L, su);
             }
           }
         }
@@ -162,12 +168,19 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
           const int32_t u = s_big[b];
           const int32_t rs = a.row[u], re = a.row[u + 1];  // checked when listed
           const int32_t su = __ldcg(sigma + u);
-          for (int64_t k = (int64_t)rs + lane; k < re; k += 32) forward_edge(a, level, sigma, order, cap, &s_tail, k, L, su);
+          for (int64_t k = (int64_t)rs + lane; k < re; k += 32) forward_edge<DEEP>(a, level, sigma, order, cap, &s_tail, k, L, su);
         }
         __syncthreads();
       }
       __syncthreads();
-      if (tid == 0) lb[L + 2] = min(s_tail, cap);
+      if (tid == 0) {
+        int32_t end = DEEP ? min(s_tail, cap) : s_tail;
+        if (!DEEP && L + 2 == kMaxLevel && end > hi) {  // level kMaxLevel may follow: an empty frontier instead
+          atomicExch(a.status + 1, 2u);
+          end = hi;
+        }
+        lb[L + 2] = end;
+      }
       __syncthreads();
       ++L;
     }
@@ -195,7 +208,7 @@ __global__ void __launch_bounds__(kThreads) bc_sources_kernel(BcArgs a) {
       __syncthreads();
     }
     // ---- leave the scratch as found: every reached vertex back to unvisited
-    const int32_t reached = min(s_tail, cap);
+    const int32_t reached = DEEP ? min(s_tail, cap) : s_tail;
     for (int32_t i = tid; i < reached; i += kThreads) {
       const int32_t v = __ldcg(order + i);
       level[v] = kMaxLevel;
@@ -228,6 +241,8 @@ constexpr int kFwdEdges = 4;      // edges per lane and step, forward
 constexpr int kBwdEdges = 2;      // ... and backward
 constexpr int kSmemBounds = 256;  // level bounds kept in shared memory; deeper ones in a.lb
 constexpr uint16_t kUnseen = 0xffff;
+constexpr int32_t kLookLevel = 11;      // levels between looks whether the call goes on
+static_assert(kMaxLevel % kLookLevel == 0, "a source looks before level kMaxLevel");
 constexpr int32_t kLongRow = 32;        // rows of at least this many edges are walked one at a time
 
 // Shared memory of a CTA of `threads` for a graph of n vertices.
@@ -301,8 +316,10 @@ __device__ __forceinline__ float ordered_sum(float du, double t, uint32_t n, int
   return du;
 }
 
+// (512 threads: 40 registers, so that three CTAs fit an SM; R-MAT 12 takes 2.6 ms with 62 and
+// two CTAs, 2.3 with three)
 template <int NT>
-__global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
+__global__ void __launch_bounds__(NT, NT == 1024 ? 1 : (NT == 512 ? 3 : 4)) bc_smem_kernel(BcArgs a) {
   constexpr int NW = NT / 32;
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ double s_dyn[];
@@ -323,6 +340,18 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
   auto set_bound = [&](int32_t L, int32_t v) {
     if (L < kSmemBounds) s_lb[L] = v;
     else lb[L] = v;
+  };
+  // Thread 0, after level L of source j, at multiples of kLookLevel: whether the source ends
+  // here, because the call takes the other kernel.  That is so when the next level, kMaxLevel,
+  // has vertices (`more`), or a quarter of the first sources is narrow.  Sources end and begin
+  // with an empty frontier then: an exit from the loops would cost each level 4 %.
+  auto leave = [&](int32_t L, int j, bool more) {
+    const bool vote = L + 1 == kLookLevel && j == (int)blockIdx.x && a.src_base == 0 && s_tail < a.narrow &&
+                        4 * (atomicAdd(a.status + 2, 1u) + 1) >= gridDim.x;
+    if (vote) atomicMax(a.status + 1, 1u);
+    if (L + 1 == kMaxLevel && more) atomicMax(a.status + 1, 2u);
+    s_stop = (n > kMaxLevel || a.narrow) && __ldcg(a.status + 1) != 0u;
+    return s_stop != 0;
   };
   // Forward edge to v from a vertex of level L with path count su (lanes with `on`).
   auto reach = [&](int32_t v, int32_t su, bool on, int32_t L) {
@@ -363,24 +392,19 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
     for (int i = tid; i < words; i += NT) seen[i] = i == src / 32 ? 1u << (src % 32) : 0u;
     if (tid == 0) {
       order[0] = (uint16_t)src;
+      s_stop = (n > kMaxLevel || a.narrow) && __ldcg(a.status + 1) != 0u;
       set_bound(0, 0);
-      set_bound(1, 1);
+      set_bound(1, s_stop ? 0 : 1);
       s_tail = 1;
       s_item[0] = s_item[1] = 0;
-      s_stop = n > kMaxLevel && __ldcg(a.status + 1) != 0u;
     }
     __syncthreads();
-    if (s_stop) return;  // another source met level kMaxLevel
     int sweep = 0;  // levels walked: the item counter of a level is reset in the next one
     // ---- forward: the frontier is order[bound(L), bound(L + 1))
     int32_t L = 0;
     for (;; ++L, ++sweep) {
       const int32_t lo = bound(L), hi = bound(L + 1);
       if (lo >= hi) break;
-      if (L == kMaxLevel) {  // the whole CTA: the bounds are the same in every thread
-        if (tid == 0) atomicExch(a.status + 1, 1u);
-        return;
-      }
       if (tid == 0) s_item[(sweep + 1) & 1] = 0;
       const int per = min(32, (hi - lo + NW - 1) / NW), items = (hi - lo + per - 1) / per;
       for (;;) {
@@ -434,11 +458,15 @@ __global__ void __launch_bounds__(NT) bc_smem_kernel(BcArgs a) {
         }
       }
       __syncthreads();
-      if (tid == 0) set_bound(L + 2, s_tail);
+      if (tid == 0) {
+        int32_t end = s_tail;
+        if ((L + 1) % kLookLevel == 0 && leave(L, j, end > hi)) end = hi;  // an empty frontier
+        set_bound(L + 2, end);
+      }
       __syncthreads();
     }
     // ---- backward: levels L - 2 down to 1 (as in bc_sources_kernel)
-    for (int32_t d = L - 2; d >= 1; --d, ++sweep) {
+    for (int32_t d = s_stop ? 0 : L - 2; d >= 1; --d, ++sweep) {
       const int32_t lo = bound(d), hi = bound(d + 1);
       if (tid == 0) s_item[(sweep + 1) & 1] = 0;
       const int per = min(32, (hi - lo + NW - 1) / NW), items = (hi - lo + per - 1) / per;
@@ -591,6 +619,30 @@ BcKernel bc_pick_smem(size_t n, int device, int* threads) {
   return bc_smem_kernel<256>;
 }
 
+// The vertices below which a source counts as narrow (BcArgs::narrow) in a call of `count`
+// sources, of which the shared-memory kernel holds `here` at once on `per_sm` CTAs per SM and
+// bc_sources_kernel `there`.  A narrow source (a grid, a chain) costs its levels' latency, not
+// its edges, so what counts is how many run at once, and state in shared memory leaves fewer:
+// the other kernel takes the call when it needs so many rounds of sources less that its
+// slower levels pay.  Its levels take 2.2 times as long on grids with one CTA per SM here, less
+// with more CTAs, more with longer rows, which it walks by a thread each (lattices of degree 4
+// / 8 / 32: 2.2 / 2.8 / 6), 3 to 6 times on random graphs just connected (degree below 2, the
+// levels of which are not as small), and as long on paths.  ms of bc_sources_kernel / shared-memory
+// kernel: 128 x 128 grid, 200 sources 2.31 / 1.92, 300 2.39 / 2.61, 2,000 5.1 / 11.6; 64 x 64
+// grid, 600 sources 1.07 / 1.00, every source 3.7 / 5.4; 5,000-vertex path, 2,000 sources 23 /
+// 52; 16,000-vertex ring, degree 32, 2,000 sources 30.6 / 32.4.  R-MAT and uniform graphs
+// have a handful of levels and never ask.
+int32_t bc_narrow_limit(int64_t n, int64_t m, int64_t count, int64_t here, int64_t there, int per_sm) {
+  auto rounds = [&](int64_t at_once) {  // between whole rounds and their share
+    const double r = (double)count / (double)at_once;
+    return r <= 1.0 ? 1.0 : 0.5 * (r + std::ceil(r));
+  };
+  const double gain = rounds(here) / rounds(there), degree = (double)m / (double)n;
+  const double slower = std::max(1.0, 2.45 - 0.25 * per_sm) * (degree < 2.0 ? 2.0 : std::max(1.0, 0.25 * degree));
+  if (gain > slower) return 32 * kLookLevel;
+  return gain > 1.0 ? 4 * kLookLevel : 0;
+}
+
 struct BcWork {
   unsigned long long ctx_id = 0;  // context the cached buffers live in (nps_context_id)
   std::mutex mu;
@@ -660,7 +712,7 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   if (!W->stream) NPS_CUDA_RETURN(cudaStreamCreateWithFlags(&W->stream, cudaStreamNonBlocking));
   if (!W->ev[0])
     for (auto& ev : W->ev) NPS_CUDA_RETURN(cudaEventCreate(&ev));
-  if (!W->status) NPS_CUDA_RETURN(cudaMalloc((void**)&W->status, 2 * sizeof(uint32_t)));
+  if (!W->status) NPS_CUDA_RETURN(cudaMalloc((void**)&W->status, 3 * sizeof(uint32_t)));
   if (!W->sms) NPS_CUDA_RETURN(cudaDeviceGetAttribute(&W->sms, cudaDevAttrMultiProcessorCount, p.device));
   cudaStream_t s = p.stream ? (cudaStream_t)p.stream : W->stream;
   if (st) memset(st, 0, sizeof(*st));
@@ -687,7 +739,7 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   }
   if (dsrc && nsrc > 0 && p.device_ptrs) {  // a bad device-side source list stops the call before any kernel reads it
     uint32_t bad = 0;
-    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 2 * sizeof(uint32_t), s));
+    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 3 * sizeof(uint32_t), s));
     bc_check_sources_kernel<<<(int)std::min<int64_t>(1024, ((int64_t)nsrc + 255) / 256), 256, 0, s>>>(dsrc, nsrc, n,
                                                                                                W->status);
     NPS_CUDA_RETURN(cudaGetLastError());
@@ -706,10 +758,11 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
   // sources shares one delta buffer
   int smem_threads = 0;
   BcKernel smem_kernel = bc_pick_smem((size_t)n, p.device, &smem_threads);
-  uint32_t h_status[2];
+  uint32_t h_status[3];
+  bool deep = false;
   int grid = 0;
   for (bool first = true;; first = false) {
-    const BcKernel kernel = smem_kernel ? smem_kernel : bc_sources_kernel;
+    const BcKernel kernel = smem_kernel ? smem_kernel : (deep ? bc_sources_kernel<true> : bc_sources_kernel<false>);
     const int threads = smem_kernel ? smem_threads : kThreads;
     const size_t dyn = smem_kernel ? bc_smem_bytes((size_t)n, threads) : 0;
     if (smem_kernel)
@@ -722,13 +775,19 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
     const int64_t by_memory = std::max<int64_t>(W->sms, (int64_t)((8ull << 30) / (per_cta * sizeof(int32_t))));
     grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>((int64_t)W->sms * std::max(1, per_sm), by_memory), count_all));
+    a.narrow = 0;
+    if (smem_kernel) {
+      int other = 0;  // CTAs of bc_sources_kernel per SM
+      NPS_CUDA_RETURN(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&other, (const void*)bc_sources_kernel<false>, kThreads, 0));
+      a.narrow = bc_narrow_limit(n, m, count_all, grid, (int64_t)W->sms * std::max(1, other), per_sm);
+    }
     if ((e = nps_ensure(&W->scratch, &W->scratch_n, per_cta * (size_t)grid, s, "bc"))) return e;
     const size_t budget = (size_t)1 << 31;  // bytes of delta rows per block
     int64_t cap = std::max<int64_t>(grid, budget / (4 * (size_t)n));
     if (p.reserved[1] > 0) cap = p.reserved[1];
     const int32_t block = (int32_t)std::max<int64_t>(1, std::min<int64_t>(count_all, cap));
     if ((e = nps_ensure(&W->delta, &W->delta_n, (size_t)block * (size_t)n, s, "bc"))) return e;
-    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 2 * sizeof(uint32_t), s));
+    NPS_CUDA_RETURN(cudaMemsetAsync(W->status, 0, 3 * sizeof(uint32_t), s));
     NPS_CUDA_RETURN(cudaMemsetAsync(dbc, 0, sizeof(float) * (size_t)n, s));
     if (smem_kernel) {
       a.level = a.sigma = a.order = nullptr;
@@ -757,8 +816,9 @@ extern "C" nps_status nps_bc(const int32_t* row_ptr, const int32_t* col, int32_t
     NPS_CUDA_RETURN(cudaMemcpyAsync(h_status, W->status, sizeof(h_status), cudaMemcpyDeviceToHost, s));
     NPS_CUDA_RETURN(cudaEventRecord(W->ev[3], s));
     NPS_CUDA_RETURN(cudaStreamSynchronize(s));
-    if (!smem_kernel || !h_status[1]) break;
-    smem_kernel = nullptr;  // levels up to kMaxLevel: again, with the kernel that counts as the reference does
+    if (!h_status[1]) break;
+    deep = h_status[1] == 2;
+    smem_kernel = nullptr;
   }
   if (st) {
     st->status = (int32_t)h_status[0];

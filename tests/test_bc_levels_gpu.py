@@ -2,11 +2,18 @@
 paths around that length, in one and in both directions, below and above the vertex count
 up to which a source fits shared memory, from one source and from several (some of them
 shallow).  Bit for bit as the oracle's restatement of bc_cpu.  A vertex on level 9999 that
-is taken more often than there is room for ends the call with an error."""
+is taken more often than there is room for ends the call with an error.  And calls of many
+sources on graphs of many small levels, which change the kernel on the way."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+def _same(a, b):
+    """Bit for bit, NaNs (0 / 0 where path counts wrap) as NaNs."""
+    a, b = np.asarray(a, np.float32), np.asarray(b, np.float32)
+    return bool(np.all((a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))))
 
 
 def _path(nps, n, both):
@@ -21,8 +28,7 @@ def test_paths(nps, oracle, cuda_device, n, both):
     g = _path(nps, n, both)
     for src in ([0], [n // 2, n - 1, 0, 7] + list(range(20, 400, 2))):
         got, st = nps.bc(g, np.array(src))
-        want = np.asarray(oracle.bc(g.row_ptr, g.col, src), np.float32)
-        assert st.status == 0 and np.array_equal(np.asarray(got, np.float32).view(np.uint32), want.view(np.uint32))
+        assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, src))
 
 
 @pytest.mark.parametrize("n,k", [(10100, 5000), (20000, 15000)])
@@ -36,5 +42,28 @@ def test_repeated_visits_end_with_an_error(nps, oracle, cuda_device, n, k):
         nps.bc(g, np.array([0]))
     assert ei.value.status == 3
     got, st = nps.bc(g, np.array([1]))  # one level less: every edge counts
-    want = np.asarray(oracle.bc(g.row_ptr, g.col, [1]), np.float32)
-    assert st.status == 0 and np.array_equal(np.asarray(got, np.float32).view(np.uint32), want.view(np.uint32))
+    assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, [1]))
+
+
+@pytest.mark.parametrize("shape,sources", [((64, 64), 0), ((3, 700), 0), ((90, 100), 500), ((17, 17), 0)])
+def test_many_sources_on_grids(nps, oracle, cuda_device, shape, sources):
+    g = nps.gen_grid(*shape, 0.05, 10, 5)
+    src = None if sources == 0 else np.linspace(0, g.n - 1, sources).astype(np.int64)
+    for block in (0, 7, 333):  # sources per block of dependency rows
+        got, st = nps.bc(g, src, nps.Params(bc_block_sources=block))
+        assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, src))
+
+
+@pytest.mark.parametrize("share", [0.05, 0.2, 0.3, 0.9])
+def test_part_of_the_sources_on_a_chain(nps, oracle, cuda_device, share):
+    """A power-law graph and a chain beside it: which kernel ends the call depends on how many
+    of the first sources lie on the chain, the result does not."""
+    core = nps.gen_rmat(11, 8, seed=3)
+    ln = 3000
+    s = np.concatenate([np.repeat(np.arange(core.n), core.degrees()), core.n + np.arange(ln - 1)])
+    d = np.concatenate([core.col, core.n + 1 + np.arange(ln - 1)])
+    g = nps.convertCSR(core.n + ln, s, d, np.ones(s.shape[0], np.uint32))
+    rng = np.random.default_rng(7)
+    src = np.where(rng.random(2500) < share, core.n + rng.integers(0, ln, 2500), rng.integers(0, core.n, 2500))
+    got, st = nps.bc(g, src)
+    assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, src))
