@@ -9,6 +9,7 @@
 // one persistent launch.  Errors come back as status codes instead of exit().
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <cmath>
@@ -817,9 +818,11 @@ nps_status ensure_pinned_wpack(nps_ctx* c, size_t bytes) {
 
 // Host-to-device copy of a graph array.  The driver moves pageable memory through its own
 // staging with one thread, about 10 GB/s; here the host's threads fill pinned slots that
-// the copy engine empties behind them.  Pinned arrays, arrays below kStageMin and a host
-// without room for the slots take the plain copy.  A call on pageable arrays, 16 cores:
-// R-MAT 18 2.0 -> 1.2 ms, R-MAT 20 8.8 -> 4.2 ms.
+// the copy engine empties behind them.  Pinned arrays, arrays below kStageMin, one host
+// thread (OMP_NUM_THREADS=1) and a host without room for the slots take the plain copy.  A
+// call on pageable arrays, plain copy / slots (ms): with 16 threads R-MAT 18 1.56 / 1.09, R-MAT
+// 20 7.9 / 3.8, with two 1.87 / 1.62 and 11.5 / 8.3; with one the slots lose, breadth-first
+// R-MAT 18 1.19 / 1.37, R-MAT 16 0.43 / 0.49.
 constexpr size_t kStageBytes = (size_t)2 << 20;
 constexpr int kStageSlots = 4;
 constexpr size_t kStageMin = (size_t)1 << 20;
@@ -841,7 +844,7 @@ bool stage_ready(nps_ctx* c) {
 
 // Whether a copy of `bytes` from or to host memory at p goes through the slots.
 bool staged(nps_ctx* c, const void* p, size_t bytes) {
-  if (bytes < kStageMin) return false;
+  if (bytes < kStageMin || omp_get_max_threads() < 2) return false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
