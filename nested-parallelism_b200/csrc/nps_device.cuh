@@ -1733,6 +1733,8 @@ static __device__ __noinline__ void cta_rounds(const InstDesc& I, Smem<BS>& sm) 
   if (S.ncnt) stage_flush(S.nbuf, S.ncnt, S.ncnt, C.qn, C.qn_tail, I.qcap, status, lane);
   if (S.fcnt) stage_flush(S.fbuf, S.fcnt, S.fcnt, C.fp, C.fp_tail, I.qcap, status, lane);
   if (S.scnt) stage_flush(S.sbuf, S.scnt, S.scnt, C.sq, C.sq_tail, I.qcap, status, lane, C.sadd);
+  // (ordered before this CTA's arrival at the team barrier by its release)
+  if (tid == 0 && sm.hop_last > 1) atomicMax(&I.ctr->hop_more[sm.hop_it % 3], sm.hop_last - 1);
   const uint32_t a[4] = {__reduce_add_sync(kFull, acc.edges), __reduce_add_sync(kFull, acc.impr),
                          __reduce_add_sync(kFull, acc.reached), __reduce_add_sync(kFull, acc.processed)};
   if (lane == 0) {
@@ -2066,8 +2068,6 @@ __device__ void solve_instance(const LaunchParams& P, const InstDesc& I, Smem<BS
       // before the barrier above, and reads it next behind the team barrier
       if (BITS && threadIdx.x == 0) sm.bits_on = 0;
       cta_rounds<BS>(I, sm);
-      // (ordered before this CTA's arrival at the team barrier by its release)
-      if (threadIdx.x == 0 && sm.hop_last > 1) atomicMax(&ctr->hop_more[it % 3], sm.hop_last - 1);
     } else {
       const uint32_t n_heavy_items = (uint32_t)((hprev_tot + (1ull << I.item_shift) - 1) >> I.item_shift);
       // vertex items hold 32 frontier entries, or 16 / 8 / 4 when the frontier is small
