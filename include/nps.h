@@ -112,7 +112,10 @@ typedef struct nps_params {
   int32_t device;           /* CUDA device ordinal */
   void* stream;             /* cudaStream_t to launch on; NULL = the library's own stream */
   double timeout_s;         /* bound on every spin wait inside the persistent kernel (default 10 s) */
-  int32_t trace;            /* 1: record one nps_trace_rec per iteration (read with nps_trace_read) */
+  int32_t trace;            /* 1: record one nps_trace_rec per iteration (read with nps_trace_read).  A
+                               traced run meets at a team barrier after every frontier: it follows no
+                               small frontier through CTA rounds and keeps no breadth-first levels in
+                               step, as a run without a trace or under the plain policy may */
   int32_t light_heavy;      /* 1 (default): with delta > 0, edges of weight >= delta are relaxed once,
                                when the bucket that settles their tail drains (Meyer-Sanders split) */
   int32_t local_rounds;     /* rounds a warp spends on the vertices it just improved before taking
@@ -140,9 +143,11 @@ typedef struct nps_params {
                                pushes (walked the next iteration; otherwise they are sorted when taken
                                from the queue and walked one iteration later).  1 = on, -1 = off,
                                0 (default) = on when the grid threshold in effect is at most
-                               NPS_SORT_AT_PUSH_AUTO_MAX edges and the edges have weights (off for
-                               nps_bfs, where every reached row is walked once anyway: R-MAT 22
-                               BFS takes 0.645 ms with it off, 0.682 ms with it on) */
+                               NPS_SORT_AT_PUSH_AUTO_MAX edges and the edges have weights.  nps_bfs
+                               reaches every row once: it sorts with 1, and with 0 where it keeps its
+                               levels in step (unordered runs on graphs of 16 M edges or more at
+                               NPS_LEVEL_GRID, 4 M at NPS_LEVEL_BLOCK and NPS_LEVEL_HYBRID), which
+                               needs every row of a level in one iteration; -1 turns both off */
   int32_t reserved2;        /* must be 0 */
 } nps_params;
 

@@ -1494,8 +1494,8 @@ __device__ __forceinline__ void walk_item(const InstDesc& I, const IterCtx& C, c
 // no stamp is needed, every improvement is followed exactly once, and the scheme stays
 // label-correcting whatever the CTAs' relative progress.  Improvements at or above the
 // bucket bound go to the far pile and processed vertices to the settle list as
-// everywhere.  Rows of at least kHopList edges go to the grid-tier list at every level
-// (the near stamp keeps each there once): the whole team walks them in the next
+// everywhere.  Rows of at least kHopList edges (or of the threshold, when that is larger) go to
+// the grid-tier list at every level (the near stamp keeps each there once): the whole team walks them in the next
 // iteration.  A CTA stops early when its queue is empty, or when it holds more than
 // kHopStop entries: enough for the whole team, so they go to the near queue like those
 // left after the last round.
@@ -1503,7 +1503,7 @@ __device__ __forceinline__ void walk_item(const InstDesc& I, const IterCtx& C, c
 // pay for it.  What bounds it: the latency of a round, about 2,800 cycles for one vertex
 // (smem entry, edges beside the distance, atomicMin beside the head's row bounds, smem
 // push).  Measured (ms before -> after): 2,000-vertex path 13.6 -> 2.7; 2048 x 2048 grid,
-// delta 16384, 47.1 -> 14.1 and 4,984 -> 301 iterations; uniform 16,384 x 131,072, delta
+// delta 16384, 47.1 -> 14.1 and 4,984 -> 301 team iterations; uniform 16,384 x 131,072, delta
 // 64, 0.318 -> 0.169; R-MAT 20 and 22 unchanged.
 // kHopEdges edges per lane (heads nb, weights in nd) of rows at distances du (kInf: the
 // row is skipped).  Every edge goes straight to its atomicMin: the distance check before

@@ -1152,7 +1152,8 @@ extern "C" nps_status nps_sssp_batch(const nps_instance* inst, int32_t count, co
     //   stage 0   a = 0, b = work (m + n): minimises the largest work / CTAs ratio;
     //   stage 1   from the first call's solve time T1 with c1 CTAs: a = iterations x
     //             kIterFloorMs (the latency floor more CTAs do not shorten),
-    //             b = (T1 - a) x c1;
+    //             b = (T1 - a) x c1 (an iteration of CTA rounds holds up to 32 frontiers
+    //             and lasts longer: a is then too low until stage 2);
     //   stage 2+  fitted through the first two calls' (c1, T1) and (c2, T2).
     constexpr double kIterFloorMs = 0.008;
     std::vector<double> fa(nteams, 0.0), fb(nteams, 0.0);

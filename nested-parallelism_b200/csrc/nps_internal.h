@@ -83,8 +83,12 @@ inline int32_t nps_policy_for(const nps_params& p, int64_t m) {
 
 // Whether a call runs the persistent kernel without the optional orderings: no
 // light/heavy split can come into effect, no degree ordering and no warp-local rounds.
-// Compiled out, they leave the item loop fewer tests and spills (512-thread CTAs,
-// R-MAT 22: plain 1.60 -> 1.53 ms, learned 1.08 -> 1.04 ms; R-MAT 20 plain 0.605 -> 0.581).
+// Compiled out, they leave the item loop fewer tests at every CTA size, and at 512 threads fewer
+// spills (154 bytes of stores instead of 170; 72 instead of 44 at 128 and 256, where it still
+// wins).  Kernel time against the general kernel, geometric means over R-MAT / uniform / grid /
+// path calls at every level: 128 threads 0.94 / 0.94 / 1.00 / 0.94, 256 0.94 / 0.95 / 0.98 /
+// 0.96, 512 0.95 / 0.98 / 1.00 / 0.99 (R-MAT 22, 512 threads: plain 1.60 -> 1.53 ms, learned 1.08
+// -> 1.04).
 inline bool nps_lean(const nps_params& p) {
   const bool split = p.light_heavy && (p.delta != 0 || p.delta_schedule != 0 || p.policy == NPS_POLICY_LEARNED);
   return !split && p.order_degree == 0 && p.local_rounds == 0;

@@ -22,7 +22,7 @@
 //          chunk sums in chunk order
 // At the WARP and BLOCK levels, rows of at least kHubRow nonzeros take the GRID
 // level's chunks too: one warp or CTA walking a hub's row outlasts everything else.
-// R-MAT scale 20, threshold 64: WARP 2.15 -> 0.54 ms, BLOCK 1.16 -> 0.47 (GRID 0.19).
+// R-MAT scale 20, threshold 64: WARP 2.12 -> 0.52 ms, BLOCK 1.16 -> 0.47 (GRID 0.18).
 //
 // Every y[r] is summed in an order fixed by the matrix alone (round by round,
 // then a fixed shuffle tree; chunk by chunk for GRID rows), so results repeat
@@ -52,7 +52,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kChunk = 1024;  // nonzeros per grid-level chunk
 // WARP and BLOCK levels: rows from kHubRow nonzeros on take grid-level chunks, in matrices of
 // at least kHubMinNnz (below, the second launch costs what a hub does: R-MAT 12 BLOCK 80 ->
-// 84 us, R-MAT 16 WARP 297 -> 163).
+// 84 us, R-MAT 16 WARP 285 -> 155).  Matrices above it without long rows pay 1 to 2.5 us for
+// that launch: uniform 60,000 x 530,000 WARP 25 -> 27 us, 1 M x 8 M 105 -> 108.
 constexpr int32_t kHubRow = 2048;
 constexpr int64_t kHubMinNnz = 1 << 19;
 constexpr int kStripes = 8;
@@ -421,7 +422,9 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_block_kernel(Mat A, int32_
 // chunk adds the row's chunk sums in chunk order.
 __global__ void __launch_bounds__(kThreads, kChunkCtas) spmv_chunks_kernel(Mat A, Lists L, double* part,
                                                                SpmvCtr* c) {
-  cudaGridDependencySynchronize();  // launched ahead of the row pass's end, which it waits for here
+  // launched as a dependent of the row pass, so that its launch is prepared beside it; it starts
+  // when the row pass has ended (with an early trigger in the row pass: no difference)
+  cudaGridDependencySynchronize();
   const uint32_t bad = c->status, nc = min((uint32_t)c->list, L.chunks);  // read together
   if (bad) return;  // the lists may have holes
   const int lane = threadIdx.x & 31;
