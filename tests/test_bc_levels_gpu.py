@@ -54,6 +54,18 @@ def test_many_sources_on_grids(nps, oracle, cuda_device, shape, sources):
         assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, src))
 
 
+@pytest.mark.parametrize("n,ctas_per_sm", [(17650, 1), (17651, 8)])
+def test_the_shared_memory_limit(nps, oracle, cuda_device, n, ctas_per_sm):
+    """The largest vertex count of the shared-memory kernel (one CTA per SM there) and the next."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = nps.gen_uniform(n, 4 * n, 10, n)
+    src = np.arange(2 * sms)
+    got, st = nps.bc(g, src)
+    assert st.status == 0 and _same(got, oracle.bc(g.row_ptr, g.col, src))
+    assert st.grid_ctas == min(ctas_per_sm, 2) * sms
+
+
 @pytest.mark.parametrize("share", [0.05, 0.2, 0.3, 0.9])
 def test_part_of_the_sources_on_a_chain(nps, oracle, cuda_device, share):
     """A power-law graph and a chain beside it: which kernel ends the call depends on how many
